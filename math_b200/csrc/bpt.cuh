@@ -363,6 +363,66 @@ struct Bpt final
                 return q.intersect_any(&n2.geometric, ray_2, distance);
         }
 
+        // What a connection's thread finds out about its line of sight: the
+        // flat and solid shapes decide, or the meshes must be asked (a ray
+        // that may enter one), or the geometric and shading normals disagree
+        // and the whole of occluded_ray() / occluded_points() is needed.
+        // The last two are answered by connect_sight_kernel.
+        enum class Sight : int
+        {
+                BLOCKED = 0,
+                OPEN = 1,
+                MESH = 2,
+                WHOLE = 3
+        };
+
+        // the ray of intersect_any() against the shapes
+        __device__ Sight shape_sight(const Vec<N, T>& normal, const Ray<N, T>& from, const T distance) const
+        {
+                Ray<N, T> ray = from;
+                ray.org = offset_ray_org(normal, from);
+                ++q.counters.queries;
+                if (q.any_shape(ray, distance))
+                {
+                        return Sight::BLOCKED;
+                }
+                return q.enters_mesh(ray, distance) ? Sight::MESH : Sight::OPEN;
+        }
+
+        // occluded_ray()
+        __device__ Sight ray_sight(const Normals<N, T>& normals, const Ray<N, T>& ray, const T distance) const
+        {
+                if (!directed_outside(dot(ray.dir, normals.shading)))
+                {
+                        return Sight::BLOCKED;
+                }
+                const T d = visibility_distance(distance);
+                if (dot(ray.dir, normals.geometric) >= 0)
+                {
+                        return shape_sight(normals.geometric, ray, d);
+                }
+                return Sight::WHOLE;
+        }
+
+        // occluded_points()
+        __device__ Sight point_sight(const Vec<N, T>& p1, const Normals<N, T>& n1, const Vec<N, T>& p2,
+                                     const Normals<N, T>& n2) const
+        {
+                const Vec<N, T> direction_1 = p2 - p1;
+                const Ray<N, T> ray_1 = Ray<N, T>::make(p1, direction_1);
+                if (!directed_outside(dot(ray_1.dir, n1.shading)) || !directed_outside(-dot(ray_1.dir, n2.shading)))
+                {
+                        return Sight::BLOCKED;
+                }
+                const bool visible_1 = dot(ray_1.dir, n1.geometric) >= 0;
+                const bool visible_2 = dot(ray_1.dir, n2.geometric) <= 0;
+                if (visible_1 && visible_2)
+                {
+                        return shape_sight(n1.geometric, ray_1, visibility_distance(direction_1.norm()));
+                }
+                return Sight::WHOLE;
+        }
+
         // -----------------------------------------------------------------
         // subpaths (bpt.cpp:60-264)
 
@@ -662,8 +722,12 @@ struct Bpt final
                 return as.usable();
         }
 
-        NBPT_CALL bool connect_light(const int t_count, const int li, const ArriveSample<N, T, C>& as,
-                                     Color<C>& out) const
+        // A strategy's contribution is formed before its line of sight is
+        // known to be open: with Sight::MESH or Sight::WHOLE the slot is
+        // written all the same, and taken back when the line turns out
+        // blocked.  BLOCKED: no contribution.
+        NBPT_CALL Sight connect_light(const int t_count, const int li, const ArriveSample<N, T, C>& as,
+                                      Color<C>& out) const
         {
                 const PathVertex<N, T, C>& cv = camera[t_count - 1];
                 const Light<N, T, C>& l = s.lights[li];
@@ -681,7 +745,7 @@ struct Bpt final
                 const T n_l = dot(cv.nrm.shading, ray_to_light.dir);
                 if (!(n_l > 0))
                 {
-                        return false;
+                        return Sight::BLOCKED;
                 }
                 BrdfTerms terms;
                 const float light_k = static_cast<float>(n_l / (as.pdf * l.distribution_pdf));
@@ -689,11 +753,12 @@ struct Bpt final
                                    as.radiance * light_k;
                 if (c.is_black())
                 {
-                        return false;
+                        return Sight::BLOCKED;
                 }
-                if (occluded_ray(cv.nrm, ray_to_light, as.distance))
+                const Sight sight = ray_sight(cv.nrm, ray_to_light, as.distance);
+                if (sight == Sight::BLOCKED)
                 {
-                        return false;
+                        return sight;
                 }
                 const float mis = static_cast<float>(mis_weight(&lv, 1, t_count));
                 out = c * mis;
@@ -708,27 +773,27 @@ struct Bpt final
                         tape.put(light_k);
                         tape.put(mis);
                 }
-                return true;
+                return sight;
         }
 
-        NBPT_CALL bool connect_strategy(const int s_count, const int t_count, Color<C>& out)
+        NBPT_CALL Sight connect_strategy(const int s_count, const int t_count, Color<C>& out)
         {
                 const PathVertex<N, T, C>& cv = camera[t_count - 1];
                 if (s_count == 0)
                 {
                         if (cv.type != static_cast<int>(VertexType::SURFACE) || cv.light < 0)
                         {
-                                return false;
+                                return Sight::BLOCKED;
                         }
                         const Light<N, T, C>& l = s.lights[cv.light];
                         if (!(dot(cv.dir, l.normal) > 0))
                         {
-                                return false;
+                                return Sight::BLOCKED;
                         }
                         const Color<C> c = l.radiance * cv.beta;
                         if (c.is_black())
                         {
-                                return false;
+                                return Sight::BLOCKED;
                         }
                         const float mis = static_cast<float>(mis_weight(light, 0, t_count));
                         out = c * mis;
@@ -740,11 +805,11 @@ struct Bpt final
                                 tape.put(cv.light);
                                 tape.put(mis);
                         }
-                        return true;
+                        return Sight::OPEN;
                 }
                 if (cv.type == static_cast<int>(VertexType::INFINITE))
                 {
-                        return false;
+                        return Sight::BLOCKED;
                 }
                 if (s_count == 1)
                 {
@@ -752,7 +817,7 @@ struct Bpt final
                         ArriveSample<N, T, C> as;
                         if (!light_arrival(t_count, li, as))
                         {
-                                return false;
+                                return Sight::BLOCKED;
                         }
                         return connect_light(t_count, li, as, out);
                 }
@@ -765,13 +830,13 @@ struct Bpt final
                 const T camera_n_l = dot(cv.nrm.shading, from_camera_to_light);
                 if (!(camera_n_l > 0))
                 {
-                        return false;
+                        return Sight::BLOCKED;
                 }
                 const Vec<N, T> light_l = -from_camera_to_light;
                 const T light_n_l = dot(lv.nrm.shading, light_l);
                 if (!(light_n_l > 0))
                 {
-                        return false;
+                        return Sight::BLOCKED;
                 }
                 BrdfTerms camera_terms;
                 BrdfTerms light_terms;
@@ -782,11 +847,12 @@ struct Bpt final
                 const Color<C> c = c0 * geometry_k;
                 if (c.is_black())
                 {
-                        return false;
+                        return Sight::BLOCKED;
                 }
-                if (occluded_points(cv.pos, cv.nrm, lv.pos, lv.nrm))
+                const Sight sight = point_sight(cv.pos, cv.nrm, lv.pos, lv.nrm);
+                if (sight == Sight::BLOCKED)
                 {
-                        return false;
+                        return sight;
                 }
                 const float mis = static_cast<float>(mis_weight(light, s_count, t_count));
                 out = c * mis;
@@ -803,7 +869,7 @@ struct Bpt final
                         tape.put(geometry_k);
                         tape.put(mis);
                 }
-                return true;
+                return sight;
         }
 
         // bpt() (bpt.cpp:267-292) after the camera subpath: BACKGROUND for a

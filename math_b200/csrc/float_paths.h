@@ -10,15 +10,17 @@
 
 #include "kernels.cuh"
 #include "pt.cuh"
+#include "walk.cuh"
 
 namespace nbpt
 {
 template <int N>
 struct FloatPathKernels final
 {
-        decltype(&paths_walk_kernel<N, float>) walk;
+        WalkKernels<N, float> walk;
         decltype(&paths_light_kernel<N, float>) light;
         decltype(&paths_connect_kernel<N, float>) connect;
+        decltype(&connect_sight_kernel<N, float>) sight;
         decltype(&paths_replay_kernel<N, float, 3, 1>) replay_rgb;
         decltype(&paths_replay_kernel<N, float, 64, 32>) replay_spectrum;
         decltype(&pt_paths_kernel<N, float, 3>) pt_rgb;

@@ -364,6 +364,24 @@ struct Simplex final
                 return (sum < 1) ? t : T(0);
         }
 
+        // intersect() without branches: every plane is loaded at once, where
+        // branches would make the loads a chain.
+        NBPT_HD T intersect_whole(const Ray<N, T>& r) const
+        {
+                const T t = plane.intersect(r);
+                const Vec<N, T> p = r.point(t);
+                bool inside = t > 0;
+                T sum = 0;
+#pragma unroll
+                for (int i = 0; i < N - 1; ++i)
+                {
+                        const T bc = planes[i].distance(p);
+                        inside = inside & (bc > 0) & (bc < 1);
+                        sum = i == 0 ? bc : sum + bc;
+                }
+                return (inside & (sum < 1)) ? t : T(0);
+        }
+
         // barycentric coordinates (hyperplane_simplex.h:70-80)
         NBPT_HD void barycentric(const Vec<N, T>& p, T* bc) const
         {

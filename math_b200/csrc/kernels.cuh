@@ -9,6 +9,7 @@
 #include "scene.cuh"
 #include "shading.cuh"
 #include "tape.cuh"
+#include "wide_bvh.cuh"
 
 #include <cooperative_groups.h>
 #include <cooperative_groups/scan.h>
@@ -207,20 +208,20 @@ struct PathsMinBlocks final
 
 // ---------------------------------------------------------------------------
 // Paths: one per pixel sample, with the random stream seed_seq{seed, pass,
-// p, i + 1}.  A chunk of pixels runs through four kernels:
-//   paths_walk_kernel     one lane per path, one bounce per iteration: the
-//                         camera and light subpaths traced with colour
-//                         channel 0 (tape.cuh), their
-//                         vertices kept in global memory, the bounce records
-//                         on the path's tape, and one task queued per
-//                         strategy with s != 1;
+// p, i + 1}.  A chunk of pixels runs through these kernels:
+//   walk_*_kernel         the camera and light subpaths traced with colour
+//                         channel 0 (tape.cuh), one wave of rays per bounce
+//                         (walk.cuh), their vertices kept in global memory
+//                         and the bounce records on the path's tape;
 //   paths_light_kernel    one thread per path: the light samples of the
 //                         s = 1 strategies in t order, since each draws from
 //                         the path's stream where the light subpath left it;
 //                         the usable ones are kept and their strategies
-//                         queued;
+//                         queued, with those of s != 1;
 //   paths_connect_kernel  one thread per queued strategy: its contribution
 //                         factors written to the strategy's tape slot;
+//   connect_sight_kernel  the lines of sight that may cross a mesh: a blocked
+//                         one clears its slot;
 //   paths_replay_kernel   the colours of all channels from the tapes.
 // Strategies of one path are independent apart from that random stream, so
 // evaluating them on separate threads changes no result; the replay sums
@@ -338,6 +339,26 @@ struct TaskQueues final
         }
 };
 
+// Reserves `n` consecutive slots of a counter for each lane of the warp with
+// one atomic; the whole warp calls it.
+__device__ inline unsigned reserve_in_warp(unsigned* const counter, const unsigned n)
+{
+        const int lane = threadIdx.x & 31;
+        unsigned sum = n;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1)
+        {
+                const unsigned x = __shfl_up_sync(0xffffffffu, sum, o);
+                sum += lane >= o ? x : 0;
+        }
+        unsigned base = 0;
+        if (lane == 31 && sum > 0)
+        {
+                base = atomicAdd(counter, sum);
+        }
+        return __shfl_sync(0xffffffffu, base, 31) + sum - n;
+}
+
 // Reserves `n` consecutive slots of a counter for each calling thread with
 // one atomic per group of threads that call it together.
 __device__ inline unsigned reserve_together(unsigned* const counter, const unsigned n)
@@ -354,152 +375,6 @@ __device__ inline unsigned reserve_together(unsigned* const counter, const unsig
         return base + before;
 }
 
-// Persistent, one bounce per iteration: every lane traces one ray and
-// processes its hit (Bpt::walk_step) in each iteration of the loop, whether
-// the ray belongs to a camera or a light subpath, so the warp's lanes run the
-// intersection and the shading together however their paths' lengths
-// differ.  A lane whose camera subpath ends starts its light subpath
-// (bpt.cpp:273-289) in the same iteration, and a lane whose path ends
-// finishes it and takes the next path from a shared counter until the chunk
-// is done.  Each path's random stream, vertices and tape are those of the
-// reference's sequential order (camera subpath, light sample, light
-// subpath).
-template <int N, typename T>
-__global__ void __launch_bounds__(128, (PathsMinBlocks<N, T>::value)) paths_walk_kernel(
-        const DeviceScene<N, T, 1> scene,
-        const long long begin,
-        const long long end,
-        const int spp,
-        const int max_depth,
-        const std::uint32_t seed,
-        const std::uint32_t pass,
-        const T* __restrict__ points,
-        PathVertex<N, T, 1>* __restrict__ vertices,
-        Pcg* __restrict__ rng,
-        std::uint32_t* __restrict__ tape,
-        const int words_per_path,
-        unsigned char* __restrict__ valid,
-        const TaskQueues queues,
-        unsigned* __restrict__ next_path,
-        PathStats* __restrict__ stats,
-        const unsigned* __restrict__ cancel)
-{
-        using B = Bpt<N, T, 1, true>;
-        using S = typename B::Subpaths;
-        const long long paths = (end - begin) * spp;
-        QueryCounters counters{0, 0, 0, 0};
-        const SceneQueries<N, T, 1> q{scene, counters};
-        Pcg g{0, 0};
-        B bpt{q, scene, g, max_depth, nullptr, nullptr};
-        typename B::Walk w;
-        Vec<N, T> gn;
-        bool from_surface = false;
-        long long i = -1; // the lane's path; -1 when it takes the next one
-        while (true)
-        {
-                if (i < 0)
-                {
-                        if (cancelled(cancel))
-                        {
-                                break; // the paths not taken keep no tape: the later kernels skip the chunk
-                        }
-                        i = reserve_together(next_path, 1);
-                        if (i >= paths)
-                        {
-                                break;
-                        }
-                        // 32-bit index arithmetic: a chunk's path index and a
-                        // screen's pixel index fit in 31 bits (the painter's chunk
-                        // limits and its screen check), and a 64-bit division costs
-                        // several times a 32-bit one
-                        const unsigned local_pixel = static_cast<unsigned>(i) / static_cast<unsigned>(spp);
-                        const int sample = static_cast<int>(static_cast<unsigned>(i) - local_pixel * spp);
-                        const unsigned p = static_cast<unsigned>(begin) + local_pixel;
-                        Vec<N - 1, T> point;
-                        {
-                                unsigned rest = p;
-#pragma unroll
-                                for (int d = 0; d < N - 1; ++d)
-                                {
-                                        const unsigned size = static_cast<unsigned>(scene.projector.size[d]);
-                                        const unsigned r = rest / size;
-                                        point[d] = static_cast<T>(static_cast<int>(rest - r * size)) +
-                                                   points[i * (N - 1) + d];
-                                        rest = r;
-                                }
-                        }
-                        const std::uint32_t words[4] = {seed, pass, static_cast<std::uint32_t>(p),
-                                                        static_cast<std::uint32_t>(sample + 1)};
-                        g = seed_seq_pcg(words, 4);
-                        bpt.camera = vertices + i * 2 * (max_depth + 1);
-                        bpt.light = bpt.camera + max_depth + 1;
-                        bpt.light_size = 0;
-                        bpt.tape.w = tape + i * static_cast<long long>(words_per_path);
-                        bpt.tape.n = TAPE_HEADER;
-                        w = bpt.camera_start(scene.projector.ray(point));
-                        from_surface = false;
-                }
-
-                Normals<N, T> normals;
-                const Hit<N, T> surface = q.scene_intersect(from_surface ? &gn : nullptr, w.ray, normals);
-                if (bpt.walk_step(w, surface, normals))
-                {
-                        gn = normals.geometric;
-                        from_surface = true;
-                        continue;
-                }
-                if (w.camera && bpt.camera_outcome() == S::CONNECT && bpt.light_start(w))
-                {
-                        from_surface = false;
-                        continue;
-                }
-
-                // the path's subpaths are done
-                const S r = bpt.camera_outcome();
-                const bool connect = r == S::CONNECT;
-                std::uint32_t* const tw = bpt.tape.w;
-                tw[0] = static_cast<std::uint32_t>(bpt.tape.n);
-                tw[1] = r != S::BACKGROUND ? 1u : 0u;
-                tw[2] = static_cast<std::uint32_t>(connect ? bpt.camera_size : 1);
-                tw[3] = static_cast<std::uint32_t>(connect ? bpt.light_size : 0);
-                valid[i] = r != S::BACKGROUND ? 1 : 0;
-                rng[i] = g;
-                if (connect)
-                {
-                        const int camera_size = bpt.camera_size;
-                        const int light_size = bpt.light_size;
-                        // s = 0 strategies: one per t
-                        unsigned k = reserve_together(&queues.count[TaskQueues::EMITTED], camera_size - 1);
-                        for (int t = 2; t <= camera_size; ++t)
-                        {
-                                queues.task(TaskQueues::EMITTED, k++) = make_task(i, t, 0);
-                        }
-                        // s >= 2 strategies
-                        unsigned task_n = 0;
-                        for (int t = 2; t <= camera_size; ++t)
-                        {
-                                for (int sc = 2; sc <= light_size; ++sc)
-                                {
-                                        task_n += (t + sc - 2 <= max_depth) ? 1 : 0;
-                                }
-                        }
-                        k = reserve_together(&queues.count[TaskQueues::CONNECT], task_n);
-                        for (int t = 2; t <= camera_size; ++t)
-                        {
-                                for (int sc = 2; sc <= light_size; ++sc)
-                                {
-                                        if (t + sc - 2 <= max_depth)
-                                        {
-                                                queues.task(TaskQueues::CONNECT, k++) = make_task(i, t, sc);
-                                        }
-                                }
-                        }
-                }
-                i = -1;
-        }
-        add_counters(counters, stats);
-}
-
 // The light sample of an s = 1 strategy (Bpt::light_arrival), kept for the
 // connect kernel.
 template <int N, typename T>
@@ -511,9 +386,78 @@ struct Arrival final
         int light;
 };
 
-// Persistent: the grid strides over the queued strategies.
+// Slots of a counter for the threads of a block that want one, in thread
+// order, with one atomic per block (a wave's list takes millions of appends,
+// which one atomic per warp on one address would bound).  Every thread of the
+// block calls it.
+template <int THREADS>
+struct BlockAppend final
+{
+        unsigned warp_count[2][THREADS / 32];
+        unsigned base[2];
+
+        __device__ void slots(unsigned* const a_counter, const bool a_want, unsigned& a_slot, unsigned* const b_counter,
+                              const bool b_want, unsigned& b_slot)
+        {
+                const int warp = threadIdx.x / 32;
+                const unsigned below = (1u << (threadIdx.x & 31)) - 1;
+                const unsigned a = __ballot_sync(0xffffffffu, a_want);
+                const unsigned b = __ballot_sync(0xffffffffu, b_want);
+                if ((threadIdx.x & 31) == 0)
+                {
+                        warp_count[0][warp] = __popc(a);
+                        warp_count[1][warp] = __popc(b);
+                }
+                __syncthreads();
+                if (threadIdx.x < 2)
+                {
+                        unsigned n = 0;
+#pragma unroll
+                        for (int w = 0; w < THREADS / 32; ++w)
+                        {
+                                const unsigned c = warp_count[threadIdx.x][w];
+                                warp_count[threadIdx.x][w] = n;
+                                n += c;
+                        }
+                        base[threadIdx.x] = n > 0 ? atomicAdd(threadIdx.x == 0 ? a_counter : b_counter, n) : 0;
+                }
+                __syncthreads();
+                a_slot = base[0] + warp_count[0][warp] + __popc(a & below);
+                b_slot = base[1] + warp_count[1][warp] + __popc(b & below);
+                __syncthreads(); // the counts are read before the next call writes them
+        }
+};
+
+// The connections whose line of sight the meshes decide (Bpt::Sight): MESH
+// from the front of one array, WHOLE from its back.
+struct SightQueue final
+{
+        std::uint32_t* tasks;
+        unsigned capacity; // one slot per strategy of the chunk
+        unsigned* count;   // [2]: MESH, WHOLE
+};
+
+// A connection's subpaths, as the connect kernels see them.
 template <int N, typename T>
-__global__ void __launch_bounds__(128, (PathsMinBlocks<N, T>::value)) paths_connect_kernel(
+__device__ inline Bpt<N, T, 1, true> connection(const SceneQueries<N, T, 1>& q, const DeviceScene<N, T, 1>& scene,
+                                                Pcg& unused, const int max_depth,
+                                                PathVertex<N, T, 1>* const vertices, std::uint32_t* const tape,
+                                                const int words_per_path, const std::uint32_t task)
+{
+        const long long i = task >> TASK_PATH_SHIFT;
+        PathVertex<N, T, 1>* const v = vertices + i * 2 * (max_depth + 1);
+        Bpt<N, T, 1, true> bpt{q, scene, unused, max_depth, v, v + max_depth + 1};
+        bpt.tape.w = tape + i * static_cast<long long>(words_per_path);
+        return bpt;
+}
+
+inline constexpr int CONNECT_THREADS = 128;
+
+// One thread per queued strategy (the grid strides over the queues): its
+// contribution factors and its line of sight past the flat and solid shapes.
+// The lines that may enter a mesh are queued for connect_sight_kernel.
+template <int N, typename T>
+__global__ void __launch_bounds__(CONNECT_THREADS) paths_connect_kernel(
         const DeviceScene<N, T, 1> scene,
         const int max_depth,
         PathVertex<N, T, 1>* __restrict__ vertices,
@@ -521,55 +465,227 @@ __global__ void __launch_bounds__(128, (PathsMinBlocks<N, T>::value)) paths_conn
         const int words_per_path,
         const Arrival<N, T>* __restrict__ arrivals,
         const TaskQueues queues,
+        const SightQueue sights,
         PathStats* __restrict__ stats)
 {
+        using S = typename Bpt<N, T, 1, true>::Sight;
+        __shared__ BlockAppend<CONNECT_THREADS> block;
         QueryCounters counters{0, 0, 0, 0};
+        const SceneQueries<N, T, 1> q{scene, counters};
         const unsigned n0 = queues.count[0];
         const unsigned n1 = queues.count[1];
         const unsigned total = n0 + n1 + queues.count[2];
-        const unsigned stride = gridDim.x * blockDim.x;
-        for (unsigned k = blockIdx.x * blockDim.x + threadIdx.x; k < total; k += stride)
+        const unsigned stride = gridDim.x * CONNECT_THREADS;
+        for (unsigned first = blockIdx.x * CONNECT_THREADS; first < total; first += stride)
         {
-                const std::uint32_t task =
-                        k < n0 ? queues.base[0][k] : (k < n0 + n1 ? queues.base[1][k - n0] : queues.base[2][k - n0 - n1]);
-                const long long i = task >> TASK_PATH_SHIFT;
-                const int t = static_cast<int>((task >> 4) & 15u);
-                const int sc = static_cast<int>(task & 15u);
-                PathVertex<N, T, 1>* const v = vertices + i * 2 * (max_depth + 1);
-                std::uint32_t* const w = tape + i * static_cast<long long>(words_per_path);
-                Pcg unused{0, 0}; // the random numbers of s = 1 were drawn by paths_light_kernel
-                const SceneQueries<N, T, 1> q{scene, counters};
-                Bpt<N, T, 1, true> bpt{q, scene, unused, max_depth, v, v + max_depth + 1};
-                bpt.camera_size = static_cast<int>(w[2]);
-                bpt.light_size = static_cast<int>(w[3]);
-                bpt.tape.w = w;
-                Color<1> c;
-                bool contributes;
-                if (sc == 1)
+                const unsigned k = first + threadIdx.x;
+                S sight = S::OPEN;
+                std::uint32_t task = 0;
+                if (k < total)
                 {
-                        const Arrival<N, T>& a = arrivals[i * max_depth + (t - 2)];
-                        ArriveSample<N, T, 1> as;
-                        as.l = a.l;
-                        as.pdf = a.pdf;
-                        as.distance = a.distance;
-                        as.radiance = scene.lights[a.light].radiance;
-                        contributes = bpt.connect_light(t, a.light, as, c);
+                        task = k < n0 ? queues.base[0][k]
+                                      : (k < n0 + n1 ? queues.base[1][k - n0] : queues.base[2][k - n0 - n1]);
+                        const int t = static_cast<int>((task >> 4) & 15u);
+                        const int sc = static_cast<int>(task & 15u);
+                        Pcg unused{0, 0}; // the random numbers of s = 1 were drawn by paths_light_kernel
+                        Bpt<N, T, 1, true> bpt = connection<N, T>(q, scene, unused, max_depth, vertices, tape,
+                                                                  words_per_path, task);
+                        std::uint32_t* const w = bpt.tape.w;
+                        Color<1> c;
+                        if (sc == 1)
+                        {
+                                const long long i = task >> TASK_PATH_SHIFT;
+                                const Arrival<N, T>& a = arrivals[i * max_depth + (t - 2)];
+                                ArriveSample<N, T, 1> as;
+                                as.l = a.l;
+                                as.pdf = a.pdf;
+                                as.distance = a.distance;
+                                as.radiance = scene.lights[a.light].radiance;
+                                sight = bpt.connect_light(t, a.light, as, c);
+                        }
+                        else
+                        {
+                                sight = bpt.connect_strategy(sc, t, c);
+                        }
+                        if (sight == S::BLOCKED)
+                        {
+                                w[tape_slot_offset(max_depth, t, sc)] = 0;
+                        }
                 }
-                else
+                unsigned mesh_slot;
+                unsigned whole_slot;
+                block.slots(sights.count, sight == S::MESH, mesh_slot, sights.count + 1, sight == S::WHOLE, whole_slot);
+                if (sight == S::MESH)
                 {
-                        contributes = bpt.connect_strategy(sc, t, c);
+                        sights.tasks[mesh_slot] = task;
                 }
-                if (!contributes)
+                else if (sight == S::WHOLE)
                 {
-                        w[tape_slot_offset(max_depth, t, sc)] = 0;
+                        sights.tasks[sights.capacity - 1 - whole_slot] = task;
                 }
+        }
+        add_counters(counters, stats);
+}
+
+// SceneQueries::intersect() for the groups that are `active`; the others'
+// `hit` stays.
+template <int N, typename T>
+__device__ inline void group_closest(const GroupQueries<N, T, 1>& group, const bool active, const Vec<N, T>& normal,
+                                     const Ray<N, T>& from, const T max_distance, Hit<N, T>& hit)
+{
+        using G = GroupQueries<N, T, 1>;
+        Ray<N, T> ray = from;
+        Hit<N, T> found;
+        found.kind = static_cast<int>(HitKind::NONE);
+        found.index = -1;
+        found.distance = max_distance;
+        if (active)
+        {
+                ray.org = offset_ray_org(normal, from);
+                group.q.counters.queries += G::lane() == 0 ? 1 : 0;
+        }
+        group.template shapes<false>(active, ray, found.distance, found.kind, found.index);
+        group.template mesh<false>(active, ray, found.distance, found.kind, found.index);
+        if (active)
+        {
+                hit = found;
+                if (hit)
+                {
+                        hit.point = group.q.hit_point(hit, ray);
+                }
+        }
+}
+
+// The line of sight of a queued connection: eight lanes each (wide_bvh.cuh).
+// A blocked line takes the strategy's contribution back.
+template <int N, typename T>
+__global__ void __launch_bounds__(CONNECT_THREADS) connect_sight_kernel(
+        const DeviceScene<N, T, 1> scene,
+        const int max_depth,
+        PathVertex<N, T, 1>* __restrict__ vertices,
+        std::uint32_t* __restrict__ tape,
+        const int words_per_path,
+        const Arrival<N, T>* __restrict__ arrivals,
+        const SightQueue sights,
+        PathStats* __restrict__ stats)
+{
+        constexpr unsigned GROUPS = CONNECT_THREADS / WIDE;
+        using B = Bpt<N, T, 1, true>;
+        using G = GroupQueries<N, T, 1>;
+        __shared__ WideStack<T> stacks[GROUPS];
+        QueryCounters counters{0, 0, 0, 0};
+        const SceneQueries<N, T, 1> q{scene, counters};
+        const G group{q, stacks[threadIdx.x / WIDE]};
+        const unsigned mesh_count = sights.count[0];
+        const unsigned count = mesh_count + sights.count[1];
+        // the warp's groups loop together
+        for (unsigned first = blockIdx.x * GROUPS + threadIdx.x / 32 * (32 / WIDE); first < count;
+             first += gridDim.x * GROUPS)
+        {
+                const unsigned m = first + threadIdx.x % 32 / WIDE;
+                const bool active = m < count;
+                const bool whole = active && m >= mesh_count;
+                std::uint32_t* slot = nullptr;
+                Ray<N, T> ray;
+                T distance = 0;
+                Vec<N, T> normal;
+                // WHOLE: the queries before the last one (occluded_points())
+                bool first_query = false;
+                bool second_query = false;
+                Ray<N, T> second;
+                Vec<N, T> second_normal;
+                if (active)
+                {
+                        const std::uint32_t task = whole ? sights.tasks[sights.capacity - 1 - (m - mesh_count)]
+                                                         : sights.tasks[m];
+                        const int t = static_cast<int>((task >> 4) & 15u);
+                        const int sc = static_cast<int>(task & 15u);
+                        Pcg unused{0, 0};
+                        const B bpt = connection<N, T>(q, scene, unused, max_depth, vertices, tape, words_per_path, task);
+                        slot = bpt.tape.w + tape_slot_offset(max_depth, t, sc);
+                        const PathVertex<N, T, 1>& cv = bpt.camera[t - 1];
+                        normal = cv.nrm.geometric;
+                        if (sc == 1)
+                        {
+                                const long long i = task >> TASK_PATH_SHIFT;
+                                const Arrival<N, T>& a = arrivals[i * max_depth + (t - 2)];
+                                ray = Ray<N, T>::make(cv.pos, a.l);
+                                distance = B::visibility_distance(a.distance);
+                                // move_and_intersect_any()
+                                second_query = whole;
+                                second = ray;
+                                second_normal = normal;
+                        }
+                        else
+                        {
+                                const PathVertex<N, T, 1>& lv = bpt.light[sc - 1];
+                                const Vec<N, T> direction = lv.pos - cv.pos;
+                                ray = Ray<N, T>::make(cv.pos, direction);
+                                distance = B::visibility_distance(direction.norm());
+                                first_query = whole && !(dot(ray.dir, cv.nrm.geometric) >= 0);
+                                second_query = whole && !(dot(ray.dir, lv.nrm.geometric) <= 0);
+                                second.org = lv.pos;
+                                second.dir = -ray.dir;
+                                second_normal = lv.nrm.geometric;
+                        }
+                }
+                bool open = !active; // decided
+                if (__any_sync(G::FULL, whole))
+                {
+                        // occluded_points(): the first query and the ray back
+                        Hit<N, T> hit;
+                        group_closest(group, first_query, normal, ray, distance, hit);
+                        if (first_query)
+                        {
+                                const T d = distance - hit.distance;
+                                open = !hit || !(d > 0);
+                                distance = d;
+                        }
+                        if (whole)
+                        {
+                                ray = second;
+                                normal = second_normal;
+                        }
+                        // move_and_intersect_any()
+                        second_query = second_query && !open;
+                        group_closest(group, second_query, normal, ray, distance, hit);
+                        if (second_query)
+                        {
+                                const T d = distance - hit.distance;
+                                open = !hit || !(d > 0);
+                                distance = d;
+                                if (!open)
+                                {
+                                        normal = q.geometric_normal(hit);
+                                        ray.org = hit.point;
+                                }
+                        }
+                }
+                if (!open)
+                {
+                        ray.org = offset_ray_org(normal, ray);
+                }
+                int kind = static_cast<int>(HitKind::NONE);
+                int index = -1;
+                if (__any_sync(G::FULL, whole && !open))
+                {
+                        counters.queries += whole && !open && G::lane() == 0 ? 1 : 0;
+                        group.template shapes<true>(whole && !open, ray, distance, kind, index);
+                }
+                group.template mesh<true>(!open, ray, distance, kind, index);
+                if (kind != static_cast<int>(HitKind::NONE) && G::lane() == 0)
+                {
+                        *slot = 0;
+                }
+                __syncwarp();
         }
         add_counters(counters, stats);
 }
 
 // One thread per path: the light samples of the s = 1 strategies, drawn in
 // t order from the path's stream where the light subpath left it; each
-// usable sample is kept and its strategy queued for the connect kernel.
+// usable sample is kept and its strategy queued for the connect kernel, with
+// the path's s = 0 and s >= 2 strategies.
 template <int N, typename T>
 __global__ void __launch_bounds__(128, (PathsMinBlocks<N, T>::value)) paths_light_kernel(
         const DeviceScene<N, T, 1> scene,
@@ -585,12 +701,14 @@ __global__ void __launch_bounds__(128, (PathsMinBlocks<N, T>::value)) paths_ligh
 {
         const long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
         unsigned queued = 0; // bit t - 2: strategy (1, t) queued
+        int camera_size = 1; // 1: no strategies
+        int light_size = 0;
         // a cancelled pass has paths without tapes (see paths_replay_kernel)
         if (i < paths && !cancelled(cancel))
         {
                 std::uint32_t* const w = tape + i * static_cast<long long>(words_per_path);
-                const int camera_size = static_cast<int>(w[2]);
-                const int light_size = static_cast<int>(w[3]);
+                camera_size = static_cast<int>(w[2]);
+                light_size = static_cast<int>(w[3]);
                 if (w[1] != 0 && light_size >= 1)
                 {
                         Pcg g = rng[i];
@@ -623,29 +741,39 @@ __global__ void __launch_bounds__(128, (PathsMinBlocks<N, T>::value)) paths_ligh
                         }
                 }
         }
-        // reserve this warp's task range with one atomic
-        const int task_n = __popc(queued);
-        const int lane = threadIdx.x & 31;
-        int offset = task_n;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1)
-        {
-                const int x = __shfl_up_sync(0xffffffffu, offset, o);
-                offset += lane >= o ? x : 0;
-        }
-        const int total = __shfl_sync(0xffffffffu, offset, 31);
-        unsigned base = 0;
-        if (lane == 31 && total > 0)
-        {
-                base = atomicAdd(&queues.count[TaskQueues::LIGHT], static_cast<unsigned>(total));
-        }
-        base = __shfl_sync(0xffffffffu, base, 31);
-        unsigned k = base + static_cast<unsigned>(offset - task_n);
+        // s = 1 strategies
+        unsigned k = reserve_in_warp(&queues.count[TaskQueues::LIGHT], __popc(queued));
         while (queued != 0)
         {
                 const int b = __ffs(queued) - 1;
                 queued &= queued - 1;
                 queues.task(TaskQueues::LIGHT, k++) = make_task(i, b + 2, 1);
+        }
+        // s = 0 strategies: one per t
+        k = reserve_in_warp(&queues.count[TaskQueues::EMITTED], camera_size - 1);
+        for (int t = 2; t <= camera_size; ++t)
+        {
+                queues.task(TaskQueues::EMITTED, k++) = make_task(i, t, 0);
+        }
+        // s >= 2 strategies
+        unsigned task_n = 0;
+        for (int t = 2; t <= camera_size; ++t)
+        {
+                for (int sc = 2; sc <= light_size; ++sc)
+                {
+                        task_n += (t + sc - 2 <= max_depth) ? 1 : 0;
+                }
+        }
+        k = reserve_in_warp(&queues.count[TaskQueues::CONNECT], task_n);
+        for (int t = 2; t <= camera_size; ++t)
+        {
+                for (int sc = 2; sc <= light_size; ++sc)
+                {
+                        if (t + sc - 2 <= max_depth)
+                        {
+                                queues.task(TaskQueues::CONNECT, k++) = make_task(i, t, sc);
+                        }
+                }
         }
 }
 

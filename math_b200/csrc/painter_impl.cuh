@@ -23,6 +23,7 @@
 #include "painter_api.h"
 #include "pt.cuh"
 #include "tables.inc"
+#include "wide_bvh.cuh"
 
 #include <cuda_runtime.h>
 
@@ -1017,6 +1018,8 @@ class SceneT final : public Scene
         DeviceArray<MeshShape<N, T>> d_meshes_;
         DeviceArray<BvhNode<N, T>> d_nodes_;
         DeviceArray<std::uint32_t> d_indices_;
+        DeviceArray<WideChild<N, T>> d_wide_;
+        DeviceArray<LeafFacet<N, T>> d_leaf_facets_;
         DeviceArray<Facet<N, T>> d_facets_;
         DeviceArray<Vec<N, T>> d_normals_;
         DeviceArray<Material<T, C>> d_materials_;
@@ -1754,6 +1757,51 @@ public:
                 bvh_builder_ = builder;
         }
 
+        // The wide nodes and the facets in leaf order of every mesh
+        // (wide_bvh.cuh), from the binary nodes.
+        void build_wide_bvhs()
+        {
+                if (meshes_.empty())
+                {
+                        return;
+                }
+                DeviceArray<std::uint32_t> parents;
+                parents.allocate(node_total_);
+                DeviceArray<std::uint32_t> wide_index;
+                wide_index.allocate(node_total_);
+                DeviceArray<unsigned> counter;
+                // the roots are the first wide nodes
+                counter.upload(std::vector<unsigned>(1, static_cast<unsigned>(meshes_.size())));
+                for (std::size_t k = 0; k < meshes_.size(); ++k)
+                {
+                        const MeshHost& m = meshes_[k];
+                        const BvhNode<N, T>* const nodes = d_nodes_.get() + m.node_offset;
+                        wide_parents_kernel<N, T><<<blocks_for(m.node_count, 128), 128>>>(
+                                nodes, m.node_count, parents.get() + m.node_offset);
+                        wide_index_kernel<N, T><<<blocks_for(m.node_count, 128), 128>>>(
+                                nodes, m.node_count, parents.get() + m.node_offset, static_cast<std::uint32_t>(k),
+                                counter.get(), wide_index.get() + m.node_offset);
+                }
+                NBPT_CUDA(cudaGetLastError());
+                unsigned count = 0;
+                counter.download(&count, 1);
+                d_wide_.allocate(static_cast<std::size_t>(count) * WIDE);
+                d_leaf_facets_.allocate(facet_total_);
+                for (const MeshHost& m : meshes_)
+                {
+                        const int facets = static_cast<int>(m.facets.size() / N);
+                        wide_children_kernel<N, T>
+                                <<<blocks_for(static_cast<long long>(m.node_count) * WIDE, 128), 128>>>(
+                                        d_nodes_.get() + m.node_offset, m.node_count, parents.get() + m.node_offset,
+                                        wide_index.get() + m.node_offset, m.index_offset, d_wide_.get());
+                        wide_facets_kernel<N, T><<<blocks_for(facets, 128), 128>>>(
+                                d_facets_.get(), d_indices_.get() + m.index_offset, facets, m.facet_offset,
+                                d_leaf_facets_.get() + m.index_offset);
+                }
+                NBPT_CUDA(cudaGetLastError());
+                NBPT_CUDA(cudaDeviceSynchronize());
+        }
+
         void finalize() override
         {
                 check_open();
@@ -2021,6 +2069,8 @@ public:
                         }
                 }
 
+                build_wide_bvhs();
+
                 // shading constants and tables
                 std::vector<T> f1(1024);
                 std::vector<T> f1a(32);
@@ -2064,6 +2114,8 @@ public:
                 device_.mesh_count = static_cast<int>(mesh_records_.size());
                 device_.nodes = d_nodes_.get();
                 device_.indices = d_indices_.get();
+                device_.wide = d_wide_.get();
+                device_.leaf_facets = d_leaf_facets_.get();
                 device_.facets = d_facets_.get();
                 device_.normals = d_normals_.get();
                 device_.materials = d_materials_.get();
@@ -2118,6 +2170,8 @@ public:
                         device_1_.mesh_count = device_.mesh_count;
                         device_1_.nodes = device_.nodes;
                         device_1_.indices = device_.indices;
+                        device_1_.wide = device_.wide;
+                        device_1_.leaf_facets = device_.leaf_facets;
                         device_1_.facets = device_.facets;
                         device_1_.normals = device_.normals;
                         device_1_.materials = d_materials_1_.get();
@@ -2208,7 +2262,8 @@ public:
         long long device_bytes() const override
         {
                 return static_cast<long long>(d_flat_.bytes() + d_solid_.bytes() + d_meshes_.bytes() + d_nodes_.bytes() +
-                                              d_indices_.bytes() + d_facets_.bytes() + d_normals_.bytes() +
+                                              d_indices_.bytes() + d_wide_.bytes() + d_leaf_facets_.bytes() +
+                                              d_facets_.bytes() + d_normals_.bytes() +
                                               d_materials_.bytes() + d_lights_.bytes());
         }
 
@@ -2275,8 +2330,11 @@ public:
 // ---------------------------------------------------------------------------
 // verification kernels
 
+// Rays of nbpt_scene_trace, eight lanes each (wide_bvh.cuh).
+inline constexpr int TRACE_THREADS = 128;
+
 template <int N, typename T, int C>
-__global__ void trace_kernel(
+__global__ void __launch_bounds__(TRACE_THREADS) trace_kernel(
         const DeviceScene<N, T, C> scene,
         const double* __restrict__ rays,
         const long long count,
@@ -2286,30 +2344,51 @@ __global__ void trace_kernel(
         double* __restrict__ t,
         double* __restrict__ point)
 {
-        const long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
-        if (i >= count)
-        {
-                return;
-        }
-        Vec<N, T> o;
-        Vec<N, T> d;
-        for (int k = 0; k < N; ++k)
-        {
-                o[k] = static_cast<T>(rays[i * 2 * N + k]);
-                d[k] = static_cast<T>(rays[i * 2 * N + N + k]);
-        }
-        const Ray<N, T> ray = Ray<N, T>::make(o, d);
+        using G = GroupQueries<N, T, C>;
+        __shared__ WideStack<T> stacks[TRACE_THREADS / WIDE];
         QueryCounters counters{0, 0, 0, 0};
         const SceneQueries<N, T, C> q{scene, counters};
+        const G group{q, stacks[threadIdx.x / WIDE]};
+        const long long i = (blockIdx.x * static_cast<long long>(TRACE_THREADS) + threadIdx.x) / WIDE;
+        const bool active = i < count;
+        Vec<N, T> o = Vec<N, T>::filled(0);
+        Vec<N, T> d = Vec<N, T>::filled(1);
+        if (active)
+        {
+                for (int k = 0; k < N; ++k)
+                {
+                        o[k] = static_cast<T>(rays[i * 2 * N + k]);
+                        d[k] = static_cast<T>(rays[i * 2 * N + N + k]);
+                }
+        }
+        const Ray<N, T> ray = Ray<N, T>::make(o, d);
+        Hit<N, T> h;
+        h.kind = static_cast<int>(HitKind::NONE);
+        h.index = -1;
+        h.distance = infinity<T>();
         if (any)
         {
-                kind[i] = q.intersect_any(nullptr, ray, infinity<T>()) ? 1 : 0;
+                group.template shapes<true>(active, ray, h.distance, h.kind, h.index);
+                group.template mesh<true>(active, ray, h.distance, h.kind, h.index);
+                if (active && G::lane() == 0)
+                {
+                        kind[i] = h ? 1 : 0;
+                }
                 return;
         }
-        const Hit<N, T> h = q.intersect(nullptr, ray, infinity<T>());
+        group.template shapes<false>(active, ray, h.distance, h.kind, h.index);
+        group.template mesh<false>(active, ray, h.distance, h.kind, h.index);
+        if (!active || G::lane() != 0)
+        {
+                return;
+        }
         kind[i] = h.kind;
         index[i] = h.index;
         t[i] = h ? static_cast<double>(h.distance) : 0.0;
+        if (h)
+        {
+                h.point = q.hit_point(h, ray);
+        }
         for (int k = 0; k < N; ++k)
         {
                 point[i * N + k] = h ? static_cast<double>(h.point[k]) : 0.0;
@@ -2508,10 +2587,14 @@ class PainterT final : public Painter
         DeviceArray<std::uint32_t> tape_;
         DeviceArray<std::uint32_t> tasks_;
         DeviceArray<unsigned> task_count_;
+        DeviceArray<unsigned char> walk_lists_;
+        DeviceArray<std::uint32_t> walk_queues_; // the mesh queue, then the light subpaths
+        DeviceArray<WalkCounters> walk_counters_;
         DeviceArray<unsigned> next_path_;
         DeviceArray<Arrival<N, T>> arrivals_;
         DeviceArray<PtEstimate> pt_estimates_;
         int connect_blocks_ = 0;
+        int walk_blocks_ = 0;
         long long launches_ = 0;
         Statistics statistics_{};
 
@@ -2549,12 +2632,13 @@ class PainterT final : public Painter
         }
 
         // device bytes of one path's buffers in a chunk (vertices, tape,
-        // random stream state, strategy tasks)
+        // random stream state, strategy tasks, walk lists)
         static long long chunk_path_bytes(const int max_depth)
         {
                 return static_cast<long long>(tape_words(max_depth)) * 4 +
                        2LL * (max_depth + 1) * sizeof(PathVertex<N, T, 1>) + sizeof(Pcg) +
-                       4LL * tape_slot_count(max_depth) + static_cast<long long>(max_depth) * sizeof(Arrival<N, T>);
+                       2 * 4LL * tape_slot_count(max_depth) + static_cast<long long>(max_depth) * sizeof(Arrival<N, T>) +
+                       WalkBuffers<N, T>::list_bytes(64) / 64 + 8;
         }
 
         // the PT kernel keeps nothing per path; its chunks only bound the
@@ -2716,8 +2800,9 @@ public:
                 {
                         tape_words_ = tape_words(max_depth_);
                         allocate_scratch();
-                        task_count_.allocate(3);
-                        next_path_.allocate(1);
+                        task_count_.allocate(5);
+                        walk_counters_.allocate(1);
+                        walk_blocks_ = sms * WALK_BLOCKS_PER_SM;
                         connect_blocks_ = sms * PathsMinBlocks<N, T>::value;
                 }
 
@@ -2764,6 +2849,7 @@ public:
                                         rgb_.bytes() +
                                         rgba_.bytes() + vertices_.bytes() + rng_.bytes() + tape_.bytes() +
                                         tasks_.bytes() + task_count_.bytes() + arrivals_.bytes() +
+                                        walk_lists_.bytes() + walk_queues_.bytes() + walk_counters_.bytes() +
                                         next_path_.bytes() + pt_estimates_.bytes();
                 return static_cast<long long>(own) + scene_->device_bytes();
         }
@@ -2776,7 +2862,7 @@ public:
         // The path kernels of this precision: single precision's come from
         // their own unit, compiled with multiply-add contraction
         // (float_paths.h); double precision's are compiled here, without it.
-        static auto walk_kernel()
+        static WalkKernels<N, T> walk_kernels()
         {
                 if constexpr (std::is_same_v<T, float>)
                 {
@@ -2784,7 +2870,7 @@ public:
                 }
                 else
                 {
-                        return &paths_walk_kernel<N, T>;
+                        return WALK_KERNELS<N, T>;
                 }
         }
         static auto light_kernel()
@@ -2807,6 +2893,17 @@ public:
                 else
                 {
                         return &paths_connect_kernel<N, T>;
+                }
+        }
+        static auto sight_kernel()
+        {
+                if constexpr (std::is_same_v<T, float>)
+                {
+                        return float_path_kernels<N>().sight;
+                }
+                else
+                {
+                        return &connect_sight_kernel<N, T>;
                 }
         }
         static auto replay_kernel()
@@ -2856,8 +2953,10 @@ public:
                 tape_.allocate(paths * tape_words_);
                 vertices_.allocate(paths * 2 * (max_depth_ + 1));
                 rng_.allocate(paths);
-                tasks_.allocate(paths * tape_slot_count(max_depth_));
+                tasks_.allocate(2 * paths * tape_slot_count(max_depth_));
                 arrivals_.allocate(paths * max_depth_);
+                walk_lists_.allocate(WalkBuffers<N, T>::list_bytes(paths));
+                walk_queues_.allocate(2 * WalkBuffers<N, T>::capacity_for(paths));
                 scratch_ready_ = true;
         }
 
@@ -2870,7 +2969,7 @@ public:
                 }
                 scratch_ready_ = false;
                 return static_cast<long long>(tape_.free() + vertices_.free() + rng_.free() + tasks_.free() +
-                                              arrivals_.free());
+                                              arrivals_.free() + walk_lists_.free() + walk_queues_.free());
         }
 
         void cancel() override
@@ -2951,7 +3050,7 @@ public:
                                         const long long e = std::min(source_first_ + sources_, b + chunk_pixels_);
                                         const long long o = b - source_first_; // the chunk in the sample arrays
                                         const long long n = (e - b) * spp_;
-                                        NBPT_CUDA(cudaMemsetAsync(task_count_.get(), 0, 3 * sizeof(unsigned), stream_));
+                                        NBPT_CUDA(cudaMemsetAsync(task_count_.get(), 0, 5 * sizeof(unsigned), stream_));
                                         // queue regions: s >= 2, then s = 1 and s = 0 (at most
                                         // max_depth each per path)
                                         TaskQueues queues;
@@ -2961,12 +3060,19 @@ public:
                                         queues.base[TaskQueues::EMITTED] =
                                                 tasks_.get() + n * (tape_slot_count(max_depth_) - max_depth_);
                                         queues.count = task_count_.get();
-                                        NBPT_CUDA(cudaMemsetAsync(next_path_.get(), 0, sizeof(unsigned), stream_));
-                                        walk_kernel()<<<std::min<long long>(connect_blocks_, blocks_for(n, 128)), 128, 0,
-                                                                  stream_>>>(
-                                                scene_1, b, e, spp_, max_depth_, seed_, pass, points_.get() + o * spp_ * (N - 1),
-                                                vertices_.get(), rng_.get(), tape_.get(), tape_words_, valid_.get() + o * spp_,
-                                                queues, next_path_.get(), stats_.get(), cancel_.get());
+                                        const SightQueue sights{tasks_.get() + n * tape_slot_count(max_depth_),
+                                                                static_cast<unsigned>(n * tape_slot_count(max_depth_)),
+                                                                task_count_.get() + 3};
+                                        NBPT_CUDA(cudaMemsetAsync(walk_counters_.get(), 0, sizeof(WalkCounters), stream_));
+                                        const long long capacity = WalkBuffers<N, T>::capacity_for(n);
+                                        const WalkBuffers<N, T> walks{walk_lists_.get(), walk_queues_.get(),
+                                                                      walk_queues_.get() + capacity,
+                                                                      walk_counters_.get(), capacity};
+                                        launches += launch_walks<N, T>(
+                                                walk_kernels(), walks, scene_1, b, n, spp_, max_depth_, seed_, pass,
+                                                points_.get() + o * spp_ * (N - 1), vertices_.get(), rng_.get(),
+                                                tape_.get(), tape_words_, valid_.get() + o * spp_, stats_.get(),
+                                                cancel_.get(), walk_blocks_, stream_);
                                         NBPT_CUDA(cudaGetLastError());
                                         light_kernel()<<<blocks_for(n, 128), 128, 0, stream_>>>(
                                                 scene_1, n, max_depth_, vertices_.get(), rng_.get(), tape_.get(), tape_words_,
@@ -2974,8 +3080,16 @@ public:
                                         NBPT_CUDA(cudaGetLastError());
                                         connect_kernel()<<<connect_blocks_, 128, 0, stream_>>>(
                                                 scene_1, max_depth_, vertices_.get(), tape_.get(), tape_words_, arrivals_.get(),
-                                                queues, stats_.get());
+                                                queues, sights, stats_.get());
                                         NBPT_CUDA(cudaGetLastError());
+                                        if (scene_1.mesh_count > 0)
+                                        {
+                                                sight_kernel()<<<walk_blocks_, 128, 0, stream_>>>(
+                                                        scene_1, max_depth_, vertices_.get(), tape_.get(), tape_words_,
+                                                        arrivals_.get(), sights, stats_.get());
+                                                NBPT_CUDA(cudaGetLastError());
+                                                launches += 1;
+                                        }
                                         constexpr int LANES = C % 32 == 0 ? 32 : 1;
                                         replay_kernel()<<<blocks_for(n * LANES, 128), 128, 0, stream_>>>(
                                                 scene_->device_materials(), scene_->device_lights(),
@@ -2983,7 +3097,7 @@ public:
                                                 tape_words_, colors_.get() + o * spp_ * C, lum_.get() + o * spp_,
                                                 scene_->cie() + 64, stats_.get(), cancel_.get());
                                         NBPT_CUDA(cudaGetLastError());
-                                        launches += 4;
+                                        launches += 3;
                                         note_progress(pass, e);
                                 }
                         }
@@ -3215,7 +3329,7 @@ void SceneT<N, T, C>::trace(
         d_t.allocate(count);
         DeviceArray<double> d_point;
         d_point.allocate(count * N);
-        trace_kernel<N, T, C><<<blocks_for(count, 128), 128>>>(s, d_rays.get(), count, any, d_kind.get(), d_index.get(),
+        trace_kernel<N, T, C><<<blocks_for(count * WIDE, TRACE_THREADS), TRACE_THREADS>>>(s, d_rays.get(), count, any, d_kind.get(), d_index.get(),
                                                                d_t.get(), d_point.get());
         NBPT_CUDA(cudaGetLastError());
         NBPT_CUDA(cudaDeviceSynchronize());
@@ -3239,7 +3353,7 @@ void SceneT<N, T, C>::trace_device(
         double* point) const
 {
         const DeviceScene<N, T, C>& s = device();
-        trace_kernel<N, T, C><<<blocks_for(count, 128), 128>>>(s, rays, count, any, kind, index, t, point);
+        trace_kernel<N, T, C><<<blocks_for(count * WIDE, TRACE_THREADS), TRACE_THREADS>>>(s, rays, count, any, kind, index, t, point);
         NBPT_CUDA(cudaGetLastError());
 }
 

@@ -10,8 +10,9 @@ template <int N>
 const FloatPathKernels<N>& float_path_kernels()
 {
         static const FloatPathKernels<N> kernels{
-                &paths_walk_kernel<N, float>,          &paths_light_kernel<N, float>,
-                &paths_connect_kernel<N, float>,       &paths_replay_kernel<N, float, 3, 1>,
+                WALK_KERNELS<N, float>,                &paths_light_kernel<N, float>,
+                &paths_connect_kernel<N, float>,       &connect_sight_kernel<N, float>,
+                &paths_replay_kernel<N, float, 3, 1>,
                 &paths_replay_kernel<N, float, 64, 32>, &pt_paths_kernel<N, float, 3>,
                 &pt_paths_kernel<N, float, 64>};
         return kernels;

@@ -9,6 +9,8 @@
 //               them out (src/geometry/accelerators/bvh.h:49-62, bvh.cpp:35-67):
 //               box, second-child or first-object offset, object count, axis
 //   indices[]   facet index per leaf slot
+//   wide[]      the same tree with eight children to a node (wide_bvh.cuh)
+//   leaf_facets[] the simplex of every leaf slot
 //   facets[]    (n-1)-simplex records (hyperplane + N-1 barycentric planes),
 //               material and vertex-normal indices
 //   normals[]   mesh vertex normals (for interpolated shading normals)
@@ -72,6 +74,36 @@ struct BvhNode final
         std::uint32_t offset; // leaf: first index slot; interior: second child
         std::uint16_t count;  // 0 for interior nodes
         std::uint16_t axis;
+};
+
+// A child of a wide node and a facet in leaf order (wide_bvh.cuh), both read
+// with 16-byte loads.
+template <int N, typename T>
+struct alignas(16) WideChild final
+{
+        T lo[N];
+        T hi[N];
+        std::uint32_t ref; // wide node, or WIDE_LEAF | first leaf slot
+        // facets of a leaf (0: a node), the slot, and the split axis of each
+        // level above the child (NO_AXIS below a leaf that ends early)
+        std::uint32_t meta;
+
+        static constexpr std::uint32_t COUNT_MASK = 0xffff;
+        static constexpr int SLOT_SHIFT = 16;
+        static constexpr std::uint32_t NO_AXIS = 7; // no ray has a sign bit there
+        static constexpr std::uint32_t UNUSED = ~0u;
+
+        NBPT_HD static constexpr int axis_shift(const int level)
+        {
+                return SLOT_SHIFT + 3 + 3 * level;
+        }
+};
+
+template <int N, typename T>
+struct alignas(16) LeafFacet final
+{
+        Simplex<N, T> simplex;
+        int facet; // global facet index
 };
 
 template <int N, typename T>
@@ -163,6 +195,8 @@ struct DeviceScene final
         int mesh_count;
         const BvhNode<N, T>* nodes;
         const std::uint32_t* indices;
+        const WideChild<N, T>* wide; // the root of mesh m is wide node m
+        const LeafFacet<N, T>* leaf_facets;
         const Facet<N, T>* facets;
         const Vec<N, T>* normals;
         const Material<T, C>* materials;
@@ -384,6 +418,63 @@ struct SceneQueries final
                 }
         }
 
+        // The flat and solid shapes of intersect(): closest hit before `best`.
+        __device__ void closest_shape(const Ray<N, T>& ray, T& best, int& kind, int& index) const
+        {
+                for (int i = 0; i < s.flat_count; ++i)
+                {
+                        ++counters.shapes;
+                        const T t = s.flat[i].shape.intersect(ray);
+                        if (t > 0 && t < best)
+                        {
+                                best = t;
+                                kind = static_cast<int>(HitKind::FLAT);
+                                index = i;
+                        }
+                }
+                for (int i = 0; i < s.solid_count; ++i)
+                {
+                        ++counters.shapes;
+                        const T t = s.solid[i].shape.intersect_volume(ray, best);
+                        if (t >= 0 && t < best)
+                        {
+                                best = t;
+                                kind = static_cast<int>(HitKind::SOLID);
+                                index = i;
+                        }
+                }
+        }
+
+        // Whether the ray enters a mesh's bound before `best` (with a
+        // smaller distance it enters no other).
+        __device__ bool enters_mesh(const Ray<N, T>& ray, const T best) const
+        {
+                for (int i = 0; i < s.mesh_count; ++i)
+                {
+                        const MeshShape<N, T>& mesh = s.meshes[i];
+                        if (!(box_volume<N>(mesh.lo, mesh.hi, ray, best) < 0))
+                        {
+                                return true;
+                        }
+                }
+                return false;
+        }
+
+        // The hit point of intersect(), from the (offset) ray.
+        __device__ Vec<N, T> hit_point(const Hit<N, T>& hit, const Ray<N, T>& ray) const
+        {
+                const Vec<N, T> p = ray.point(hit.distance);
+                switch (static_cast<HitKind>(hit.kind))
+                {
+                case HitKind::FLAT:
+                        return s.flat[hit.index].shape.plane.project(p);
+                case HitKind::SOLID:
+                        return s.solid[hit.index].shape.project(p);
+                default:
+                        return s.facets[hit.index].simplex.plane.project(p);
+                }
+        }
+
         // Closest hit of the ray against every shape with t < max_distance,
         // after moving the origin off the surface it leaves
         // (scene.cpp:70-95, 97-123, 161-178).
@@ -456,6 +547,30 @@ struct SceneQueries final
                         break;
                 }
                 return hit;
+        }
+
+        // The flat and solid shapes of intersect_any().
+        __device__ bool any_shape(const Ray<N, T>& ray, const T max_distance) const
+        {
+                for (int i = 0; i < s.flat_count; ++i)
+                {
+                        ++counters.shapes;
+                        const T t = s.flat[i].shape.intersect(ray);
+                        if (t > 0 && t < max_distance)
+                        {
+                                return true;
+                        }
+                }
+                for (int i = 0; i < s.solid_count; ++i)
+                {
+                        ++counters.shapes;
+                        const T t = s.solid[i].shape.intersect_volume(ray, max_distance);
+                        if (t >= 0 && t < max_distance)
+                        {
+                                return true;
+                        }
+                }
+                return false;
         }
 
         // Any hit with t < max_distance (scene.cpp:125-133, 180-189).

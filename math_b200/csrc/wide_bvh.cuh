@@ -1,0 +1,448 @@
+// The BVH as the path kernels traverse it: eight children to a node, a ray to
+// eight lanes.
+//
+// A wide node holds the descendants of a binary node (scene.cuh, BvhNode)
+// three levels below it, or its leaves where the tree ends earlier; the
+// facets' hyperplanes are stored a second time in leaf order.  Eight lanes
+// test a node's children together, then a leaf's facets.
+//
+// The traversal makes the binary traversal's decisions, so it finds the same
+// facet at the same distance bit for bit, equal distances included:
+//   - A box lies inside its parent's, and the slab test is monotone in the
+//     bounds under rounding, so a ray that misses the parent misses the box:
+//     the intermediate boxes need no test.
+//   - Children are visited in the binary order: at each of the levels between
+//     the side the ray's sign on the split axis asks for comes first.
+//   - A box test against a distance d is near <= min(d, far), near and far
+//     not depending on d; the binary traversal tests a box when it reaches
+//     it, so a stacked child keeps its near, which is compared with the
+//     distance of that moment.
+//   - Of a leaf's facets the closest one hit wins, the first of several at
+//     that distance, as when they are tested one by one.
+//
+// Why: rays that enter a mesh's box visit 79 binary nodes and 8 facets on
+// average on the 4-space hull of 20,000 points, 209 and 35 on a 5-space hull
+// of 6,000 points, where the longest of 100,000 visits 1,483 and 411.  One
+// lane per ray walked those as a chain of dependent loads: a launch lasted as
+// long as its longest ray (2.4 ms in 5-space, 0.6 to 1.1 ms in 4-space,
+// whatever the number of rays), with the other lanes of its warp idle.
+#pragma once
+
+#include "scene.cuh"
+
+namespace nbpt
+{
+inline constexpr int WIDE_LEVELS = 3;
+inline constexpr int WIDE = 1 << WIDE_LEVELS;
+inline constexpr std::uint32_t WIDE_LEAF = 1u << 31;
+
+// Entries of a ray's stack: a node leaves at most WIDE - 1 children behind
+// per level of wide nodes.
+inline constexpr int WIDE_STACK = ((host::BVH_MAX_DEPTH + WIDE_LEVELS - 1) / WIDE_LEVELS) * (WIDE - 1) + 1;
+
+// ---------------------------------------------------------------------------
+// build, from the binary nodes of one mesh
+
+template <int N, typename T>
+__global__ void wide_parents_kernel(const BvhNode<N, T>* __restrict__ nodes, const int count,
+                                    std::uint32_t* __restrict__ parents)
+{
+        const int i = static_cast<int>(blockIdx.x * blockDim.x + threadIdx.x);
+        if (i >= count)
+        {
+                return;
+        }
+        if (i == 0)
+        {
+                parents[0] = ~0u;
+        }
+        if (nodes[i].count == 0)
+        {
+                parents[i + 1] = static_cast<std::uint32_t>(i);
+                parents[nodes[i].offset] = static_cast<std::uint32_t>(i);
+        }
+}
+
+// The wide node of every binary node that becomes one: the root (`root`) and
+// the interior nodes at depths that are multiples of WIDE_LEVELS.
+template <int N, typename T>
+__global__ void wide_index_kernel(const BvhNode<N, T>* __restrict__ nodes, const int count,
+                                  const std::uint32_t* __restrict__ parents, const std::uint32_t root,
+                                  unsigned* __restrict__ counter, std::uint32_t* __restrict__ wide_index)
+{
+        const int i = static_cast<int>(blockIdx.x * blockDim.x + threadIdx.x);
+        if (i >= count)
+        {
+                return;
+        }
+        if (i == 0)
+        {
+                wide_index[0] = root;
+                return;
+        }
+        if (nodes[i].count != 0)
+        {
+                return;
+        }
+        int depth = 0;
+        for (std::uint32_t p = parents[i]; p != ~0u; p = parents[p])
+        {
+                ++depth;
+        }
+        if (depth % WIDE_LEVELS == 0)
+        {
+                wide_index[i] = atomicAdd(counter, 1u);
+        }
+}
+
+// One thread per child slot of every binary node that becomes a wide one.
+template <int N, typename T>
+__global__ void wide_children_kernel(const BvhNode<N, T>* __restrict__ nodes, const int count,
+                                     const std::uint32_t* __restrict__ parents,
+                                     const std::uint32_t* __restrict__ wide_index, const int index_offset,
+                                     WideChild<N, T>* __restrict__ children)
+{
+        const long long thread = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
+        const int i = static_cast<int>(thread / WIDE);
+        const unsigned slot = static_cast<unsigned>(thread % WIDE);
+        if (i >= count)
+        {
+                return;
+        }
+        if (i != 0)
+        {
+                if (nodes[i].count != 0)
+                {
+                        return;
+                }
+                int depth = 0;
+                for (std::uint32_t p = parents[i]; p != ~0u; p = parents[p])
+                {
+                        ++depth;
+                }
+                if (depth % WIDE_LEVELS != 0)
+                {
+                        return;
+                }
+        }
+        WideChild<N, T> c;
+        std::uint32_t at = static_cast<std::uint32_t>(i);
+        unsigned meta = slot << WideChild<N, T>::SLOT_SHIFT;
+        bool used = true;
+        for (int level = 0; level < WIDE_LEVELS; ++level)
+        {
+                const int bit = WIDE_LEVELS - 1 - level;
+                if (nodes[at].count != 0)
+                {
+                        // a leaf above the last level: in the first slot below it
+                        used = used && (slot & ((2u << bit) - 1)) == 0;
+                        meta |= WideChild<N, T>::NO_AXIS << WideChild<N, T>::axis_shift(level);
+                        continue;
+                }
+                meta |= static_cast<unsigned>(nodes[at].axis) << WideChild<N, T>::axis_shift(level);
+                at = ((slot >> bit) & 1u) != 0 ? nodes[at].offset : at + 1;
+        }
+        const BvhNode<N, T>& n = nodes[at];
+#pragma unroll
+        for (int d = 0; d < N; ++d)
+        {
+                // an unused slot's box is never hit
+                c.lo[d] = used ? n.lo[d] : infinity<T>();
+                c.hi[d] = used ? n.hi[d] : -infinity<T>();
+        }
+        c.ref = n.count != 0 ? (WIDE_LEAF | (index_offset + n.offset)) : wide_index[at];
+        c.meta = used ? (meta | n.count) : WideChild<N, T>::UNUSED;
+        children[static_cast<long long>(wide_index[i]) * WIDE + slot] = c;
+}
+
+// The facet of every leaf slot of one mesh.
+template <int N, typename T>
+__global__ void wide_facets_kernel(const Facet<N, T>* __restrict__ facets, const std::uint32_t* __restrict__ indices,
+                                   const int count, const int facet_offset, LeafFacet<N, T>* __restrict__ out)
+{
+        const int i = static_cast<int>(blockIdx.x * blockDim.x + threadIdx.x);
+        if (i >= count)
+        {
+                return;
+        }
+        const int f = static_cast<int>(indices[i]) + facet_offset;
+        LeafFacet<N, T> r;
+        r.simplex = facets[f].simplex;
+        r.facet = f;
+        out[i] = r;
+}
+
+// ---------------------------------------------------------------------------
+// queries: eight lanes per ray.  Every lane of the warp calls them, with its
+// group's ray; `active` and the results are equal in a group's lanes.
+
+template <typename T>
+struct WideStack final
+{
+        T near[WIDE_STACK];
+        std::uint32_t ref[WIDE_STACK];
+        std::uint32_t facets[WIDE_STACK];
+};
+
+template <int N, typename T, int C>
+struct GroupQueries final
+{
+        static constexpr unsigned FULL = 0xffffffffu;
+
+        const SceneQueries<N, T, C>& q;
+        WideStack<T>& stack; // the group's, in shared memory
+
+        __device__ static unsigned lane()
+        {
+                return threadIdx.x % WIDE;
+        }
+
+        __device__ static unsigned group_shift()
+        {
+                return threadIdx.x % 32 / WIDE * WIDE;
+        }
+
+        // The flat and solid shapes of SceneQueries::intersect(), a shape to
+        // a lane: the closest hit before `best`, the first of several at one
+        // distance; (ANY) whether there is one, in `kind`.
+        template <bool ANY>
+        __device__ void shapes(const bool active, const Ray<N, T>& ray, T& best, int& kind, int& index) const
+        {
+                const DeviceScene<N, T, C>& s = q.s;
+                T t = best;
+                int shape = -1; // in the order of the tests: flat shapes, then solid ones
+                if (active)
+                {
+                        for (int i = static_cast<int>(lane()); i < s.flat_count + s.solid_count; i += WIDE)
+                        {
+                                ++q.counters.shapes;
+                                if (i < s.flat_count)
+                                {
+                                        const T x = s.flat[i].shape.intersect(ray);
+                                        if (x > 0 && x < t)
+                                        {
+                                                t = x;
+                                                shape = i;
+                                        }
+                                }
+                                else
+                                {
+                                        const T x = s.solid[i - s.flat_count].shape.intersect_volume(ray, t);
+                                        if (x >= 0 && x < t)
+                                        {
+                                                t = x;
+                                                shape = i;
+                                        }
+                                }
+                        }
+                }
+#pragma unroll
+                for (int o = 1; o < WIDE; o <<= 1)
+                {
+                        const T x = __shfl_xor_sync(FULL, t, o);
+                        const int i = __shfl_xor_sync(FULL, shape, o);
+                        if (i >= 0 && (shape < 0 || x < t || (x == t && i < shape)))
+                        {
+                                t = x;
+                                shape = i;
+                        }
+                }
+                if (shape >= 0)
+                {
+                        const bool flat = shape < s.flat_count;
+                        kind = static_cast<int>(flat ? HitKind::FLAT : HitKind::SOLID);
+                        if constexpr (!ANY)
+                        {
+                                best = t;
+                                index = flat ? shape : shape - s.flat_count;
+                        }
+                }
+        }
+
+        // The meshes of SceneQueries::intersect(): the closest hit before
+        // `best`, or (ANY) whether there is one, in `kind`.
+        template <bool ANY>
+        __device__ void mesh(const bool active, const Ray<N, T>& ray, T& best, int& kind, int& index) const
+        {
+                const DeviceScene<N, T, C>& s = q.s;
+                Vec<N, T> rec;
+                unsigned neg = 0;
+#pragma unroll
+                for (int i = 0; i < N; ++i)
+                {
+                        rec[i] = (ray.dir[i] == 0) ? infinity<T>() : (1 / ray.dir[i]);
+                        if (ray.dir[i] < 0)
+                        {
+                                neg |= 1u << i;
+                        }
+                }
+                for (int m = 0; m < s.mesh_count; ++m)
+                {
+                        // the mesh's bound is its root box entry (shapes/mesh.cpp:225-229)
+                        const bool enters = active && !(ANY && kind != static_cast<int>(HitKind::NONE)) &&
+                                            !(box_volume<N>(s.meshes[m].lo, s.meshes[m].hi, ray, best) < 0);
+                        if (!__any_sync(FULL, enters))
+                        {
+                                continue;
+                        }
+                        int top = 0;
+                        if (enters)
+                        {
+                                top = 1;
+                                if (lane() == 0)
+                                {
+                                        stack.near[0] = 0;
+                                        stack.ref[0] = static_cast<std::uint32_t>(m);
+                                }
+                        }
+                        __syncwarp();
+                        while (__any_sync(FULL, top > 0))
+                        {
+                                bool node = false;
+                                bool leaf = false;
+                                std::uint32_t ref = 0;
+                                int facets = 0;
+                                while (top > 0 && !node && !leaf)
+                                {
+                                        --top;
+                                        if (stack.near[top] <= best)
+                                        {
+                                                ref = stack.ref[top];
+                                                leaf = (ref & WIDE_LEAF) != 0;
+                                                node = !leaf;
+                                                facets = leaf ? static_cast<int>(stack.facets[top]) : 0;
+                                        }
+                                }
+                                __syncwarp(); // the entry is read before it is written again
+                                if (__any_sync(FULL, node))
+                                {
+                                        children(node, ref, ray, rec, neg, best, top);
+                                }
+                                if (__any_sync(FULL, leaf))
+                                {
+                                        leaf_facets<ANY>(facets, ref & ~WIDE_LEAF, ray, best, kind, index, top);
+                                }
+                        }
+                }
+        }
+
+private:
+        // Tests the children of node `ref` and stacks those that are hit, the
+        // first to visit on top.
+        __device__ void children(const bool node, const std::uint32_t ref, const Ray<N, T>& ray, const Vec<N, T>& rec,
+                                 const unsigned neg, const T distance, int& top) const
+        {
+                using W = WideChild<N, T>;
+                bool hit = false;
+                T near = 0;
+                unsigned key = 0;
+                W c;
+                if (node)
+                {
+                        c = q.s.wide[static_cast<long long>(ref) * WIDE + lane()];
+                        T far = distance;
+#pragma unroll
+                        for (int i = 0; i < N; ++i)
+                        {
+                                const bool negative = (neg >> i) & 1u;
+                                const T a1 = ((negative ? c.hi[i] : c.lo[i]) - ray.org[i]) * rec[i];
+                                const T a2 = ((negative ? c.lo[i] : c.hi[i]) - ray.org[i]) * rec[i];
+                                near = a1 > near ? a1 : near;
+                                far = a2 < far ? a2 : far;
+                        }
+                        if (c.meta != W::UNUSED)
+                        {
+                                ++q.counters.nodes;
+                                hit = !(far < near);
+                        }
+                        // the place in the binary visiting order
+                        key = (c.meta >> W::SLOT_SHIFT) & (WIDE - 1);
+#pragma unroll
+                        for (int level = 0; level < WIDE_LEVELS; ++level)
+                        {
+                                const unsigned axis = (c.meta >> W::axis_shift(level)) & W::NO_AXIS;
+                                key ^= ((neg >> axis) & 1u) << (WIDE_LEVELS - 1 - level);
+                        }
+                }
+                const unsigned hits =
+                        (__reduce_or_sync(FULL, hit ? 1u << (group_shift() + key) : 0u) >> group_shift()) & 0xffu;
+                const int count = __popc(hits);
+                if (top + count > WIDE_STACK)
+                {
+                        // the builders refuse trees this deep; end the query
+                        // rather than write past the stack
+                        q.counters.overflows += lane() == 0 ? 1 : 0;
+                        top = 0;
+                }
+                else
+                {
+                        if (hit)
+                        {
+                                const int at = top + __popc(hits >> (key + 1));
+                                stack.near[at] = near;
+                                stack.ref[at] = c.ref;
+                                stack.facets[at] = c.meta & W::COUNT_MASK;
+                        }
+                        top += count;
+                }
+                __syncwarp();
+        }
+
+        template <bool ANY>
+        __device__ void leaf_facets(const int count, const std::uint32_t slot, const Ray<N, T>& ray, T& best, int& kind,
+                                    int& index, int& top) const
+        {
+                for (int first = 0; __any_sync(FULL, first < count); first += WIDE)
+                {
+                        const int k = first + static_cast<int>(lane());
+                        T t = infinity<T>();
+                        int facet = -1;
+                        bool hit = false;
+                        if (k < count)
+                        {
+                                ++q.counters.facets;
+                                const LeafFacet<N, T> f = q.s.leaf_facets[static_cast<long long>(slot) + k];
+                                const T x = f.simplex.intersect_whole(ray);
+                                if (x > 0 && x < best)
+                                {
+                                        t = x;
+                                        facet = f.facet;
+                                        hit = true;
+                                }
+                        }
+                        const unsigned hits = (__ballot_sync(FULL, hit) >> group_shift()) & 0xffu;
+                        if constexpr (ANY)
+                        {
+                                if (hits != 0)
+                                {
+                                        kind = static_cast<int>(HitKind::FACET);
+                                        top = 0;
+                                }
+                        }
+                        else
+                        {
+                                // the closest of the group's hits, the first of several
+                                int winner = 0;
+                                T closest = t;
+#pragma unroll
+                                for (int i = 0; i < WIDE; ++i)
+                                {
+                                        const T x = __shfl_sync(FULL, t, i, WIDE);
+                                        if (i == 0 || x < closest)
+                                        {
+                                                closest = x;
+                                                winner = i;
+                                        }
+                                }
+                                const int f = __shfl_sync(FULL, facet, winner, WIDE);
+                                if (hits != 0)
+                                {
+                                        best = closest;
+                                        kind = static_cast<int>(HitKind::FACET);
+                                        index = f;
+                                }
+                        }
+                }
+        }
+};
+} // namespace nbpt
