@@ -17,8 +17,8 @@
 // partial_sort perform, sources are merged into a receiving pixel in
 // increasing pixel index, and all sums are in float as the reference keeps
 // them.  From the same samples the image is therefore the reference's, bit
-// for bit.  One thread gathers for one receiving pixel, so no atomics are
-// needed.
+// for bit.  Every receiving pixel is gathered by its own thread or warp, so
+// no atomics are needed.
 //
 // The same merges run with the radiance and weight sums in double (the sum
 // type S of the sets): the single-precision trace keeps its per-pixel sums
@@ -338,13 +338,13 @@ NBPT_HD void merge_colors_with_sum(const SetView<C, S>& a, const SetView<C, S>& 
         out = r;
 }
 
-// Merge a fresh group into a pixel's colour set (samples/merge.cpp:198-223).
+// Merge a fresh group, or the set of one, into a pixel's colour set
+// (samples/merge.cpp:198-223).
 template <int C, typename S>
-NBPT_HD void merge_color_group(ColorSet<C, S>& s, const ColorGroup<C>& g, const S* g_sum, const S g_wsum,
-                               const bool g_full)
+NBPT_HD void merge_color_view(ColorSet<C, S>& s, const SetView<C, S>& b, const S* g_sum, const S g_wsum,
+                              const bool g_full)
 {
         const SetView<C, S> a{&s, nullptr, 0};
-        const SetView<C, S> b{nullptr, &g, g_full ? 1 : 0};
         const int a_count = a.count();
         const int b_count = b.count();
         if (a_count + b_count > HELD_OUT)
@@ -404,34 +404,50 @@ NBPT_HD void merge_color_group(ColorSet<C, S>& s, const ColorGroup<C>& g, const 
         s = r;
 }
 
-// Background sets: the same merges on weights only.
-template <typename S>
-NBPT_HD void merge_background_group(BackgroundSet<S>& s, const float* gw, const int n)
+template <int C, typename S>
+NBPT_HD void merge_color_group(ColorSet<C, S>& s, const ColorGroup<C>& g, const S* g_sum, const S g_wsum,
+                               const bool g_full)
 {
-        // gw: the group's weights, already ordered (order_group on values)
-        const bool g_full = n > HELD_OUT;
-        float held[HELD_OUT];
-        S g_sum = 0;
-        int g_count = n;
-        if (g_full)
+        merge_color_view<C, S>(s, SetView<C, S>{nullptr, &g, g_full ? 1 : 0}, g_sum, g_wsum, g_full);
+}
+
+// Background sets: the same merges on weights only.
+//
+// The set of a group of `n` background weights, weight(k) in order
+// (order_group on values).
+template <typename S, typename Weight>
+NBPT_HD void background_group(BackgroundSet<S>& g, const int n, const Weight& weight)
+{
+        g.weight_sum = 0;
+        g.count = n;
+        g.full = n > HELD_OUT ? 1 : 0;
+        if (g.full)
         {
-                held[0] = gw[0];
-                held[1] = gw[1];
+                g.weights[0] = weight(0);
+                g.weights[1] = weight(1);
                 for (int k = 2; k < n - 2; ++k)
                 {
-                        g_sum += gw[k];
+                        g.weight_sum += weight(k);
                 }
-                held[2] = gw[n - 2];
-                held[3] = gw[n - 1];
-                g_count = HELD_OUT;
+                g.weights[2] = weight(n - 2);
+                g.weights[3] = weight(n - 1);
+                g.count = HELD_OUT;
+                return;
         }
-        else
+        for (int k = 0; k < n; ++k)
         {
-                for (int k = 0; k < n; ++k)
-                {
-                        held[k] = gw[k];
-                }
+                g.weights[k] = weight(k);
         }
+}
+
+// Merges a group's set into a pixel's.
+template <typename S>
+NBPT_HD void merge_background(BackgroundSet<S>& s, const BackgroundSet<S>& g)
+{
+        const bool g_full = g.full != 0;
+        const float* const held = g.weights;
+        const S g_sum = g.weight_sum;
+        const int g_count = g.count;
         const int a_count = s.full ? HELD_OUT : s.count;
         if (a_count + g_count > HELD_OUT)
         {
@@ -579,8 +595,16 @@ NBPT_HD void merge_background_group(BackgroundSet<S>& s, const float* gw, const 
         s.full = 0;
 }
 
+template <typename S>
+NBPT_HD void merge_background_group(BackgroundSet<S>& s, const float* gw, const int n)
+{
+        BackgroundSet<S> g;
+        background_group(g, n, [&](const int k) { return gw[k]; });
+        merge_background(s, g);
+}
+
 // ---------------------------------------------------------------------------
-// accumulation kernel: one thread per receiving pixel
+// accumulation
 
 template <int N>
 struct Screen final
@@ -593,12 +617,78 @@ struct Screen final
         long long source_first = 0;
 };
 
-// Merge one pass's samples of the 3^(n-1) neighbours into receiving pixel t
-// (global index).
-template <int N, typename T, int C, typename S>
-NBPT_HD void accumulate_pixel(
-        const Screen<N>& screen,
-        const long long t,
+// RGB accumulation in two kernels: the group of every (source pixel,
+// receiving pixel) pair is formed by a thread of its own (group_kernel), then
+// every receiving pixel merges its groups in increasing source index
+// (merge_groups_kernel).
+//
+// Forming the groups is nearly all of the work (spp weights of N - 1 filter
+// factors each, their ordering and sums, 3^(N-1) times per pixel) and its
+// pairs are independent; one thread per pixel did them one after the other,
+// which left most of the GPU idle on small screens (4,096 pixels of 81
+// samples in 5-space: 10.3 ms) and repeated every factor 3^(N-2) times.  The
+// threads of a block share a few sources: a source's factors (three offsets
+// per sample and axis) are computed once into shared memory, and a warp's
+// lanes read the same samples of the same source.  A group travels as a
+// sample set (120-152 bytes).
+
+inline constexpr int neighbours(const int n)
+{
+        return n == 3 ? 9 : (n == 4 ? 27 : 81);
+}
+
+// threads of a group_kernel block and the source pixels they share
+template <int N>
+struct GroupShape final
+{
+        static constexpr int THREADS = N == 5 ? 256 : 128;
+        static constexpr int SOURCES = THREADS / neighbours(N);
+
+        // dynamic shared memory for `sources` source pixels: the filter
+        // factors and the samples' order (one byte each, by thread)
+        template <typename T>
+        static constexpr std::size_t bytes(const int sources, const int spp)
+        {
+                return static_cast<std::size_t>(spp) * (sources * (N - 1) * 3 * sizeof(T) + THREADS);
+        }
+
+        // as many sources as fit in a quarter of an SM's shared memory, at
+        // least one (256 samples of 5-space double precision: 87 KB)
+        template <typename T>
+        static constexpr int sources(const int spp)
+        {
+                int s = SOURCES;
+                while (s > 1 && bytes<T>(s, spp) > 56 * 1024)
+                {
+                        --s;
+                }
+                return s;
+        }
+};
+
+// A thread's column of the shared order array.
+struct OrderColumn final
+{
+        unsigned char* p;
+        int stride;
+
+        NBPT_HD unsigned char& operator[](const int i) const
+        {
+                return p[i * stride];
+        }
+};
+
+// The groups of the source pixels [source_begin, source_begin +
+// source_count) for the receiving pixels [begin, begin + count) (global
+// indices); groups: [count][3^(N-1)].
+template <int N, typename T, typename S>
+__global__ void __launch_bounds__(GroupShape<N>::THREADS) group_kernel(
+        const Screen<N> screen,
+        const long long begin,
+        const long long count,
+        const long long source_begin,
+        const long long source_count,
+        const int sources, // per block
         const int spp,
         const T* __restrict__ points,
         const float* __restrict__ colors,
@@ -606,11 +696,182 @@ NBPT_HD void accumulate_pixel(
         const unsigned char* __restrict__ valid,
         const T alpha,
         const T exp_radius,
-        PixelState<C, S>& st)
+        PixelState<3, S>* __restrict__ groups)
 {
+        constexpr int NB = neighbours(N);
+        constexpr int THREADS = GroupShape<N>::THREADS;
+        constexpr int C = 3;
+        extern __shared__ __align__(16) unsigned char group_shared[];
+        T* const factors = reinterpret_cast<T*>(group_shared); // [source][sample][axis][offset]
+        unsigned char* const orders =
+                group_shared + static_cast<std::size_t>(sources) * spp * (N - 1) * 3 * sizeof(T); // [sample][thread]
+
+        // pixel_filter.h:57-69, gaussian.h:66-77: the factor of an axis for
+        // the receiving pixel one below, at, and one above the source
+        const long long first = static_cast<long long>(blockIdx.x) * sources;
+        const long long sample_first = (source_begin + first - screen.source_first) * spp;
+        const int here = static_cast<int>(min(static_cast<long long>(sources), source_count - first));
+        for (int e = threadIdx.x; e < here * spp * (N - 1); e += THREADS)
+        {
+                const T v = points[sample_first * (N - 1) + e];
+#pragma unroll
+                for (int o = 0; o < 3; ++o)
+                {
+                        const T x = (static_cast<T>(o - 1) + T(0.5)) - v;
+                        factors[e * 3 + o] = max_value(T(0), exp(alpha * x * x) - exp_radius);
+                }
+        }
+        __syncthreads();
+
+        const int local = threadIdx.x / NB;
+        const int nb = threadIdx.x % NB;
+        if (local >= here)
+        {
+                return;
+        }
+        const long long p = source_begin + first + local;
+        // the source is neighbour nb of the receiving pixel: digit d of nb is
+        // its offset + 1 along axis d
+        long long t = 0;
+        int at[N - 1]; // the factors' offsets
+        {
+                int tc[N - 1];
+                long long rest = p;
+                int digits = nb;
+                bool inside = true;
+#pragma unroll
+                for (int d = 0; d < N - 1; ++d)
+                {
+                        const int digit = digits % 3;
+                        digits /= 3;
+                        tc[d] = static_cast<int>(rest % screen.size[d]) - digit + 1;
+                        rest /= screen.size[d];
+                        inside = inside && tc[d] >= 0 && tc[d] < screen.size[d];
+                        at[d] = d * 3 + 2 - digit;
+                }
+                if (!inside)
+                {
+                        return;
+                }
+#pragma unroll
+                for (int d = N - 2; d >= 0; --d)
+                {
+                        t = t * screen.size[d] + tc[d];
+                }
+        }
+        if (t < begin || t >= begin + count)
+        {
+                return;
+        }
+
+        const long long sample = (p - screen.source_first) * spp;
+        const T* const mine = factors + static_cast<std::size_t>(local) * spp * (N - 1) * 3;
+        const auto weight = [&](const int j)
+        {
+                const T* const f = mine + j * ((N - 1) * 3);
+                T w = f[at[0]];
+#pragma unroll
+                for (int d = 1; d < N - 1; ++d)
+                {
+                        w *= f[at[d]];
+                }
+                return w;
+        };
+        const auto weight_float = [&](const int j) { return static_cast<float>(weight(j)); };
+
+        // the selection of colour and background samples (com/select.h:28-47):
+        // colour samples from the front of the column, background from its back
+        const OrderColumn order{orders + threadIdx.x, THREADS};
+        const OrderColumn order_bg{orders + (spp - 1) * THREADS + threadIdx.x, -THREADS};
+        int nc = 0;
+        int nbg = 0;
+        for (int j = 0; j < spp; ++j)
+        {
+                if (!(weight(j) > 0))
+                {
+                        continue;
+                }
+                if (valid[sample + j])
+                {
+                        order[nc++] = static_cast<unsigned char>(j);
+                }
+                else
+                {
+                        order_bg[nbg++] = static_cast<unsigned char>(j);
+                }
+        }
+        PixelState<C, S>& out = groups[(t - begin) * NB + nb];
+        out.color.count = nc < HELD_OUT ? nc : HELD_OUT;
+        out.color.full = nc > HELD_OUT ? 1 : 0;
+        out.background.count = nbg < HELD_OUT ? nbg : HELD_OUT;
+        if (nc > 0)
+        {
+                order_group(order, nc, [&](const int j) { return weight_float(j) * lum[sample + j]; });
+                const float* const c = colors + sample * C;
+                S sum[C] = {0, 0, 0};
+                S wsum = 0;
+                // create_with_sum (samples/com/create.h:28-55)
+                for (int k = HELD_OUT / 2; k < nc - HELD_OUT / 2 && nc > HELD_OUT; ++k)
+                {
+                        const int j = order[k];
+                        const float w = weight_float(j);
+#pragma unroll
+                        for (int i = 0; i < C; ++i)
+                        {
+                                sum[i] += w * c[j * C + i];
+                        }
+                        wsum += w;
+                }
+#pragma unroll
+                for (int i = 0; i < C; ++i)
+                {
+                        out.color.color_sum[i] = sum[i];
+                }
+                out.color.weight_sum = wsum;
+                for (int k = 0; k < HELD_OUT && k < nc; ++k)
+                {
+                        const int j = order[nc > HELD_OUT && k >= HELD_OUT / 2 ? nc - HELD_OUT + k : k];
+                        const float w = weight_float(j);
+#pragma unroll
+                        for (int i = 0; i < C; ++i)
+                        {
+                                out.color.colors[k][i] = w * c[j * C + i];
+                        }
+                        out.color.weights[k] = w;
+                        out.color.contributions[k] = w * lum[sample + j];
+                }
+        }
+        if (nbg > 0)
+        {
+                // background samples are ordered by value
+                order_group(order_bg, nbg, weight_float);
+                BackgroundSet<S> g;
+                background_group(g, nbg, [&](const int k) { return weight_float(order_bg[k]); });
+                out.background = g;
+        }
+}
+
+// One thread per receiving pixel: its groups merged in increasing source
+// index (the last screen axis outermost).
+inline constexpr int MERGE_THREADS = 32;
+
+template <int N, typename S>
+__global__ void __launch_bounds__(MERGE_THREADS) merge_groups_kernel(
+        const Screen<N> screen,
+        const long long begin, // of the receiving pixels, global index
+        const long long count,
+        const PixelState<3, S>* __restrict__ groups,
+        PixelState<3, S>* __restrict__ state) // of the pixels from `begin` on
+{
+        constexpr int NB = neighbours(N);
+        const long long i = blockIdx.x * static_cast<long long>(MERGE_THREADS) + threadIdx.x;
+        if (i >= count)
+        {
+                return;
+        }
         int tc[N - 1];
         {
-                long long rest = t;
+                long long rest = begin + i;
 #pragma unroll
                 for (int d = 0; d < N - 1; ++d)
                 {
@@ -618,144 +879,35 @@ NBPT_HD void accumulate_pixel(
                         rest /= screen.size[d];
                 }
         }
-
-        float w[MAX_GROUP];
-        float contribution[MAX_GROUP];
-        int color_order[MAX_GROUP];
-        float background[MAX_GROUP];
-
-        int neighbours = 1;
-#pragma unroll
-        for (int d = 0; d < N - 1; ++d)
+        PixelState<3, S> st = state[i];
+        for (int nb = 0; nb < NB; ++nb)
         {
-                neighbours *= 3;
-        }
-        // sources in increasing pixel index: the last screen axis outermost
-        for (int nb = 0; nb < neighbours; ++nb)
-        {
-                int pc[N - 1];
+                int rest = nb;
                 bool inside = true;
-                {
-                        int rest = nb;
 #pragma unroll
-                        for (int d = 0; d < N - 1; ++d)
-                        {
-                                pc[d] = tc[d] + (rest % 3) - 1;
-                                rest /= 3;
-                                inside = inside && pc[d] >= 0 && pc[d] < screen.size[d];
-                        }
+                for (int d = 0; d < N - 1; ++d)
+                {
+                        const int pc = tc[d] + rest % 3 - 1;
+                        rest /= 3;
+                        inside = inside && pc >= 0 && pc < screen.size[d];
                 }
                 if (!inside)
                 {
                         continue;
                 }
-                long long p = 0;
-#pragma unroll
-                for (int d = N - 2; d >= 0; --d)
+                const PixelState<3, S>& group = groups[i * NB + nb];
+                if (group.color.count > 0)
                 {
-                        p = p * screen.size[d] + pc[d];
+                        const ColorSet<3, S> g = group.color;
+                        merge_color_view<3, S>(st.color, SetView<3, S>{&g, nullptr, 0}, g.color_sum, g.weight_sum,
+                                               g.full != 0);
                 }
-
-                // weights (pixel_filter.h:57-69, gaussian.h:66-77) and the
-                // selection of colour and background samples (com/select.h:28-47)
-                int nc = 0;
-                int nbg = 0;
-                for (int j = 0; j < spp; ++j)
+                if (group.background.count > 0)
                 {
-                        const long long sidx = (p - screen.source_first) * spp + j;
-                        const T x0 = (static_cast<T>(tc[0] - pc[0]) + T(0.5)) - points[sidx * (N - 1)];
-                        T weight = max_value(T(0), exp(alpha * x0 * x0) - exp_radius);
-#pragma unroll
-                        for (int d = 1; d < N - 1; ++d)
-                        {
-                                const T x = (static_cast<T>(tc[d] - pc[d]) + T(0.5)) - points[sidx * (N - 1) + d];
-                                weight *= max_value(T(0), exp(alpha * x * x) - exp_radius);
-                        }
-                        if (!(weight > 0))
-                        {
-                                continue;
-                        }
-                        const float wf = static_cast<float>(weight);
-                        if (valid[sidx])
-                        {
-                                w[j] = wf;
-                                contribution[j] = wf * lum[sidx];
-                                color_order[nc++] = j;
-                        }
-                        else
-                        {
-                                background[nbg++] = wf;
-                        }
-                }
-
-                if (nc > 0)
-                {
-                        order_group(color_order, nc, [&](const int i) { return contribution[i]; });
-                        const ColorGroup<C> g{colors + (p - screen.source_first) * spp * C, w, contribution, color_order, nc, C, 1, 0};
-                        S g_sum[C];
-                        S g_wsum = 0;
-#pragma unroll 8
-                        for (int c = 0; c < C; ++c)
-                        {
-                                g_sum[c] = 0;
-                        }
-                        const bool g_full = nc > HELD_OUT;
-                        if (g_full)
-                        {
-                                // create_with_sum (samples/com/create.h:28-55)
-                                for (int k = HELD_OUT / 2; k < nc - HELD_OUT / 2; ++k)
-                                {
-#pragma unroll 8
-                                        for (int c = 0; c < C; ++c)
-                                        {
-                                                g_sum[c] += g.color(k, c);
-                                        }
-                                        g_wsum += w[color_order[k]];
-                                }
-                        }
-                        merge_color_group(st.color, g, g_sum, g_wsum, g_full);
-                }
-                if (nbg > 0)
-                {
-                        // background samples are ordered by value
-                        int order[MAX_GROUP];
-                        for (int k = 0; k < nbg; ++k)
-                        {
-                                order[k] = k;
-                        }
-                        order_group(order, nbg, [&](const int i) { return background[i]; });
-                        float sorted[MAX_GROUP];
-                        for (int k = 0; k < nbg; ++k)
-                        {
-                                sorted[k] = background[order[k]];
-                        }
-                        merge_background_group(st.background, sorted, nbg);
+                        merge_background(st.background, group.background);
                 }
         }
-}
-
-// accumulation kernel: one thread per receiving pixel, no atomics
-template <int N, typename T, int C, typename S>
-__global__ void __launch_bounds__(128) accumulate_kernel(
-        const Screen<N> screen,
-        const long long pixel_count,
-        const int spp,
-        const T* __restrict__ points,
-        const float* __restrict__ colors,
-        const float* __restrict__ lum,
-        const unsigned char* __restrict__ valid,
-        const T alpha,
-        const T exp_radius,
-        PixelState<C, S>* __restrict__ state)
-{
-        const long long t = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
-        if (t >= pixel_count)
-        {
-                return;
-        }
-        PixelState<C, S> st = state[t];
-        accumulate_pixel<N, T, C, S>(screen, screen.first + t, spp, points, colors, lum, valid, alpha, exp_radius, st);
-        state[t] = st;
+        state[i] = st;
 }
 
 // Spectral colours: one warp per receiving pixel.  The lanes compute the

@@ -11,10 +11,10 @@ inline constexpr int HELD_OUT = 4; // the reference's FILTER_SAMPLE_COUNT (pixel
 // ---------------------------------------------------------------------------
 // ordering of a group: the steps of libstdc++'s insertion sort (for up to
 // eight entries) and of its binary-heap partial selection (more entries), on
-// an index array.
+// an index array (a pointer, or anything indexed like one).
 
-template <typename Less>
-NBPT_HD void insertion_sort(int* a, const int n, const Less& less)
+template <typename Array, typename Less>
+NBPT_HD void insertion_sort(Array a, const int n, const Less& less)
 {
         for (int i = 1; i < n; ++i)
         {
@@ -50,8 +50,8 @@ NBPT_HD void insertion_sort(int* a, const int n, const Less& less)
 // the top's place in the array, and the new heap is {x on top, s} when s < x,
 // else {s on top, x}; sort_heap leaves s, t.  The entries between keep the
 // order these moves give them, the order the reference sums them in.
-template <typename Key>
-NBPT_HD void order_group(int* a, const int n, const Key& key)
+template <typename Array, typename Key>
+NBPT_HD void order_group(Array a, const int n, const Key& key)
 {
         if (n <= 1)
         {

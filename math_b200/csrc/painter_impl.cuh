@@ -94,6 +94,15 @@ public:
                 }
         }
 
+        // keeps a buffer that is large enough
+        void allocate_if_smaller(const std::size_t n)
+        {
+                if (size_ < n)
+                {
+                        allocate(n);
+                }
+        }
+
         void upload(const std::vector<X>& v)
         {
                 allocate(v.size());
@@ -2570,6 +2579,7 @@ class PainterT final : public Painter
         }
         DeviceArray<PixelState<C, float>> state_;    // float sums
         DeviceArray<PixelState<C, double>> state64_; // double sums
+        DeviceArray<unsigned char> groups_;          // accumulate_groups()
         DeviceArray<PathStats> stats_;
         DeviceArray<unsigned> cancel_; // nonzero: the passes take no more paths
         bool scratch_ready_ = false;   // the per-chunk path buffers are allocated
@@ -2585,10 +2595,8 @@ class PainterT final : public Painter
         DeviceArray<PathVertex<N, T, 1>> vertices_;
         DeviceArray<Pcg> rng_;
         DeviceArray<std::uint32_t> tape_;
-        DeviceArray<std::uint32_t> tasks_;
+        DeviceArray<unsigned char> queues_; // queue_bytes()
         DeviceArray<unsigned> task_count_;
-        DeviceArray<unsigned char> walk_lists_;
-        DeviceArray<std::uint32_t> walk_queues_; // the mesh queue, then the light subpaths
         DeviceArray<WalkCounters> walk_counters_;
         DeviceArray<unsigned> next_path_;
         DeviceArray<Arrival<N, T>> arrivals_;
@@ -2596,6 +2604,7 @@ class PainterT final : public Painter
         int connect_blocks_ = 0;
         int walk_blocks_ = 0;
         long long launches_ = 0;
+        int launches_accumulate_ = 0;
         Statistics statistics_{};
 
         // Device memory for the per-path buffers of one chunk.  The walk and
@@ -2631,14 +2640,22 @@ class PainterT final : public Painter
 #endif
         }
 
+        // The strategy queues of a chunk (the tasks, then the lines of sight
+        // left to the meshes), in whose place the walks keep their lists and
+        // queues before there are strategies.
+        static long long queue_bytes(const long long paths, const int max_depth)
+        {
+                return std::max(2 * 4LL * tape_slot_count(max_depth) * paths,
+                                WalkBuffers<N, T>::list_bytes(paths) + 8 * WalkBuffers<N, T>::capacity_for(paths));
+        }
+
         // device bytes of one path's buffers in a chunk (vertices, tape,
-        // random stream state, strategy tasks, walk lists)
+        // random stream state, strategy queues)
         static long long chunk_path_bytes(const int max_depth)
         {
                 return static_cast<long long>(tape_words(max_depth)) * 4 +
                        2LL * (max_depth + 1) * sizeof(PathVertex<N, T, 1>) + sizeof(Pcg) +
-                       2 * 4LL * tape_slot_count(max_depth) + static_cast<long long>(max_depth) * sizeof(Arrival<N, T>) +
-                       WalkBuffers<N, T>::list_bytes(64) / 64 + 8;
+                       queue_bytes(64, max_depth) / 64 + static_cast<long long>(max_depth) * sizeof(Arrival<N, T>);
         }
 
         // the PT kernel keeps nothing per path; its chunks only bound the
@@ -2671,6 +2688,28 @@ public:
                        (pixel_sums == PIXEL_SUMS_DEFAULT && std::is_same_v<T, float>);
         }
 
+        // The scratch of accumulate_groups(): all receiving pixels of most
+        // renders, and for a larger screen ranges long enough that the sources
+        // that two ranges share are few (5-space: 43,000 pixels, of which a
+        // range shares those of its first and last rows).
+        static constexpr long long GROUP_BYTES = 512LL << 20;
+
+        template <typename S>
+        static long long group_pixels(const long long pixels)
+        {
+                return std::min(pixels, GROUP_BYTES / static_cast<long long>(neighbours(N) * sizeof(PixelState<3, S>)));
+        }
+
+        static long long group_bytes(const long long pixels, const bool sums_in_double)
+        {
+                if constexpr (C != 3)
+                {
+                        return 0;
+                }
+                return sums_in_double ? group_pixels<double>(pixels) * neighbours(N) * sizeof(PixelState<3, double>)
+                                      : group_pixels<float>(pixels) * neighbours(N) * sizeof(PixelState<3, float>);
+        }
+
         // device bytes a painter of these parameters allocates
         static long long estimate_bytes(const long long pixels, const int spp, const int max_depth, const int strata,
                                         const Integrator integrator, const long long budget = 0,
@@ -2685,7 +2724,7 @@ public:
                                                 : chunk_pixels(pixels, spp, max_depth, integrator, budget) * spp *
                                                           chunk_path_bytes(max_depth);
                 return (strata + 1) * sizeof(T) + samples * per_sample + pixels * per_pixel + sizeof(PathStats) +
-                       chunk;
+                       chunk + group_bytes(pixels, sums_in_double);
         }
 
         // slab_end < 0: the whole screen; else the rows [slab_begin, slab_end)
@@ -2776,6 +2815,7 @@ public:
                 {
                         state_.allocate(pixels_);
                 }
+                groups_.allocate(group_bytes(pixels_, double_sums_));
                 stats_.allocate(1);
                 NBPT_CUDA(cudaMemsetAsync(stats_.get(), 0, sizeof(PathStats), stream_));
                 cancel_.allocate(1);
@@ -2846,10 +2886,10 @@ public:
         {
                 const std::size_t own = offsets_.bytes() + points_.bytes() + colors_.bytes() + lum_.bytes() +
                                         valid_.bytes() + state_.bytes() + state64_.bytes() + stats_.bytes() +
-                                        rgb_.bytes() +
+                                        rgb_.bytes() + groups_.bytes() +
                                         rgba_.bytes() + vertices_.bytes() + rng_.bytes() + tape_.bytes() +
-                                        tasks_.bytes() + task_count_.bytes() + arrivals_.bytes() +
-                                        walk_lists_.bytes() + walk_queues_.bytes() + walk_counters_.bytes() +
+                                        queues_.bytes() + task_count_.bytes() + arrivals_.bytes() +
+                                        walk_counters_.bytes() +
                                         next_path_.bytes() + pt_estimates_.bytes();
                 return static_cast<long long>(own) + scene_->device_bytes();
         }
@@ -2953,10 +2993,8 @@ public:
                 tape_.allocate(paths * tape_words_);
                 vertices_.allocate(paths * 2 * (max_depth_ + 1));
                 rng_.allocate(paths);
-                tasks_.allocate(2 * paths * tape_slot_count(max_depth_));
+                queues_.allocate(queue_bytes(paths, max_depth_));
                 arrivals_.allocate(paths * max_depth_);
-                walk_lists_.allocate(WalkBuffers<N, T>::list_bytes(paths));
-                walk_queues_.allocate(2 * WalkBuffers<N, T>::capacity_for(paths));
                 scratch_ready_ = true;
         }
 
@@ -2968,8 +3006,8 @@ public:
                         return 0;
                 }
                 scratch_ready_ = false;
-                return static_cast<long long>(tape_.free() + vertices_.free() + rng_.free() + tasks_.free() +
-                                              arrivals_.free() + walk_lists_.free() + walk_queues_.free());
+                return static_cast<long long>(tape_.free() + vertices_.free() + rng_.free() + queues_.free() +
+                                              arrivals_.free() + groups_.free());
         }
 
         void cancel() override
@@ -3017,6 +3055,7 @@ public:
                         NBPT_CUDA(cudaGetLastError());
                         NBPT_CUDA(cudaEventRecord(ev_paths_, stream_));
                         long long launches = 2;
+                        launches_accumulate_ = 0;
                         DeviceScene<N, T, 1> scene_1 = scene_->device_channel_0();
                         scene_1.flat_shading = flat_shading_ ? 1 : 0;
                         if (integrator_ == Integrator::PT)
@@ -3054,19 +3093,21 @@ public:
                                         // queue regions: s >= 2, then s = 1 and s = 0 (at most
                                         // max_depth each per path)
                                         TaskQueues queues;
-                                        queues.base[TaskQueues::CONNECT] = tasks_.get();
+                                        std::uint32_t* const tasks = reinterpret_cast<std::uint32_t*>(queues_.get());
+                                        queues.base[TaskQueues::CONNECT] = tasks;
                                         queues.base[TaskQueues::LIGHT] =
-                                                tasks_.get() + n * (tape_slot_count(max_depth_) - 2 * max_depth_);
+                                                tasks + n * (tape_slot_count(max_depth_) - 2 * max_depth_);
                                         queues.base[TaskQueues::EMITTED] =
-                                                tasks_.get() + n * (tape_slot_count(max_depth_) - max_depth_);
+                                                tasks + n * (tape_slot_count(max_depth_) - max_depth_);
                                         queues.count = task_count_.get();
-                                        const SightQueue sights{tasks_.get() + n * tape_slot_count(max_depth_),
+                                        const SightQueue sights{tasks + n * tape_slot_count(max_depth_),
                                                                 static_cast<unsigned>(n * tape_slot_count(max_depth_)),
                                                                 task_count_.get() + 3};
                                         NBPT_CUDA(cudaMemsetAsync(walk_counters_.get(), 0, sizeof(WalkCounters), stream_));
                                         const long long capacity = WalkBuffers<N, T>::capacity_for(n);
-                                        const WalkBuffers<N, T> walks{walk_lists_.get(), walk_queues_.get(),
-                                                                      walk_queues_.get() + capacity,
+                                        std::uint32_t* const walk_queues = reinterpret_cast<std::uint32_t*>(
+                                                queues_.get() + WalkBuffers<N, T>::list_bytes(n));
+                                        const WalkBuffers<N, T> walks{queues_.get(), walk_queues, walk_queues + capacity,
                                                                       walk_counters_.get(), capacity};
                                         launches += launch_walks<N, T>(
                                                 walk_kernels(), walks, scene_1, b, n, spp_, max_depth_, seed_, pass,
@@ -3123,7 +3164,7 @@ public:
                         }
                         NBPT_CUDA(cudaGetLastError());
                         NBPT_CUDA(cudaEventRecord(ev_end_, stream_));
-                        launches_ = launches;
+                        launches_ = launches + std::max(0, launches_accumulate_ - 1);
                 }
                 passes_done_ += passes;
         }
@@ -3195,9 +3236,52 @@ public:
                 }
                 else
                 {
-                        accumulate_kernel<N, T, C, S><<<blocks_for(pixels_, 128), 128, 0, stream_>>>(
-                                screen, pixels_, spp_, points_.get(), colors_.get(), lum_.get(), valid_.get(), alpha,
-                                exp_radius, state);
+                        static_assert(C == 3);
+                        accumulate_groups(screen, alpha, exp_radius, state);
+                }
+        }
+
+        // RGB: the groups of a range of receiving pixels at a time, as many
+        // as the scratch holds (GROUP_BYTES); the sources of a range reach one
+        // pixel past it along every axis.
+        template <typename S>
+        void accumulate_groups(const Screen<N>& screen, const T alpha, const T exp_radius,
+                               PixelState<3, S>* const state)
+        {
+                using Shape = GroupShape<N>;
+                const long long range = group_pixels<S>(pixels_);
+                // given back by release_scratch()
+                groups_.allocate_if_smaller(group_bytes(pixels_, double_sums_));
+                auto* const groups = reinterpret_cast<PixelState<3, S>*>(groups_.get());
+                long long reach = 0;
+                long long row = 1;
+                for (int d = 0; d < N - 1; ++d)
+                {
+                        reach += row;
+                        row *= screen.size[d];
+                }
+                const int sources = Shape::template sources<T>(spp_);
+                const std::size_t shared = Shape::template bytes<T>(sources, spp_);
+                if (shared > 48 * 1024)
+                {
+                        NBPT_CUDA(cudaFuncSetAttribute(group_kernel<N, T, S>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                       static_cast<int>(shared)));
+                }
+                for (long long b = first_; b < first_ + pixels_; b += range)
+                {
+                        const long long n = std::min(range, first_ + pixels_ - b);
+                        const long long source_begin = std::max(source_first_, b - reach);
+                        const long long source_end = std::min(source_first_ + sources_, b + n + reach);
+                        const long long source_count = source_end - source_begin;
+                        group_kernel<N, T, S>
+                                <<<static_cast<unsigned>((source_count + sources - 1) / sources), Shape::THREADS, shared,
+                                   stream_>>>(screen, b, n, source_begin, source_count, sources, spp_, points_.get(),
+                                              colors_.get(), lum_.get(), valid_.get(), alpha, exp_radius, groups);
+                        NBPT_CUDA(cudaGetLastError());
+                        merge_groups_kernel<N, S><<<blocks_for(n, MERGE_THREADS), MERGE_THREADS, 0, stream_>>>(
+                                screen, b, n, groups, state + (b - first_));
+                        NBPT_CUDA(cudaGetLastError());
+                        launches_accumulate_ += 2;
                 }
         }
 
