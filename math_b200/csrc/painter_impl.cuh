@@ -2603,6 +2603,7 @@ class PainterT final : public Painter
         DeviceArray<PtEstimate> pt_estimates_;
         int connect_blocks_ = 0;
         int walk_blocks_ = 0;
+        int sms_ = 0;
         long long launches_ = 0;
         int launches_accumulate_ = 0;
         Statistics statistics_{};
@@ -2827,6 +2828,7 @@ public:
                 NBPT_CUDA(cudaGetDevice(&device));
                 device_ = device;
                 NBPT_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
+                sms_ = sms;
                 chunk_pixels_ = chunk_pixels(sources_, spp_, max_depth_, integrator_, chunk_budget_);
                 if (integrator_ == Integrator::PT)
                 {
@@ -3241,6 +3243,17 @@ public:
                 }
         }
 
+        // dynamic shared memory beyond 48 KB has to be asked for
+        template <typename Kernel>
+        static void allow_shared(Kernel* const kernel, const std::size_t bytes)
+        {
+                if (bytes > 48 * 1024)
+                {
+                        NBPT_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                       static_cast<int>(bytes)));
+                }
+        }
+
         // RGB: the groups of a range of receiving pixels at a time, as many
         // as the scratch holds (GROUP_BYTES); the sources of a range reach one
         // pixel past it along every axis.
@@ -3249,6 +3262,18 @@ public:
                                PixelState<3, S>* const state)
         {
                 using Shape = GroupShape<N>;
+                if (SmallScreen<N>::template fits<S>(pixels_, spp_, sms_))
+                {
+                        const std::size_t shared = SmallScreen<N>::template bytes<S>(spp_);
+                        allow_shared(accumulate_small_kernel<N, T, S>, shared);
+                        accumulate_small_kernel<N, T, S>
+                                <<<blocks_for(pixels_, SmallScreen<N>::PIXELS), Shape::THREADS, shared, stream_>>>(
+                                        screen, pixels_, spp_, points_.get(), colors_.get(), lum_.get(), valid_.get(),
+                                        alpha, exp_radius, state);
+                        NBPT_CUDA(cudaGetLastError());
+                        launches_accumulate_ = 1;
+                        return;
+                }
                 const long long range = group_pixels<S>(pixels_);
                 // given back by release_scratch()
                 groups_.allocate_if_smaller(group_bytes(pixels_, double_sums_));
@@ -3262,11 +3287,7 @@ public:
                 }
                 const int sources = Shape::template sources<T>(spp_);
                 const std::size_t shared = Shape::template bytes<T>(sources, spp_);
-                if (shared > 48 * 1024)
-                {
-                        NBPT_CUDA(cudaFuncSetAttribute(group_kernel<N, T, S>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                       static_cast<int>(shared)));
-                }
+                allow_shared(group_kernel<N, T, S>, shared);
                 for (long long b = first_; b < first_ + pixels_; b += range)
                 {
                         const long long n = std::min(range, first_ + pixels_ - b);
