@@ -14,6 +14,8 @@
 #include "shading.cuh"
 #include "tape.cuh"
 
+#include <type_traits>
+
 namespace nbpt
 {
 // Longest subpath: MAX_DEPTH + 1 vertices for a maximum depth of 8.
@@ -27,8 +29,9 @@ enum class VertexType : int
         INFINITE = 3
 };
 
+// Read and written with 16-byte accesses.
 template <int N, typename T, int C>
-struct PathVertex final
+struct alignas(16) PathVertex final
 {
         int type;
         int material; // surface
@@ -234,7 +237,7 @@ struct Bpt final
         }
 
         // compute_pdf (vertex_pdf.h:141-190)
-        NBPT_CALL T compute_pdf(const PathVertex<N, T, C>& prev, const PathVertex<N, T, C>& v,
+        __device__ __forceinline__ T compute_pdf(const PathVertex<N, T, C>& prev, const PathVertex<N, T, C>& v,
                                  const PathVertex<N, T, C>& next) const
         {
                 Vec<N, T> to_prev;
@@ -264,7 +267,7 @@ struct Bpt final
         }
 
         // compute_light_pdf (vertex_pdf.h:88-115)
-        NBPT_CALL T compute_light_pdf(const PathVertex<N, T, C>& lv, const PathVertex<N, T, C>& next) const
+        __device__ __forceinline__ T compute_light_pdf(const PathVertex<N, T, C>& lv, const PathVertex<N, T, C>& next) const
         {
                 if (lv.type == static_cast<int>(VertexType::LIGHT))
                 {
@@ -470,8 +473,11 @@ struct Bpt final
         // walk goes on.  The reference intersects the next ray of the last
         // bounce as well and never uses the hit; the walk ends there instead,
         // with the same vertices, random stream and tape.
-        NBPT_CALL bool walk_step(Walk& w, const Hit<N, T>& surface, const Normals<N, T>& normals)
+        __device__ __forceinline__ bool walk_step(Walk& w, const Hit<N, T>& surface_in, const Normals<N, T>& normals_in)
         {
+                Hit<N, T> surface = surface_in;
+                surface.point = opaque(surface_in.point);
+                const Normals<N, T> normals{opaque(normals_in.geometric), opaque(normals_in.shading)};
                 PathVertex<N, T, C>* const path = w.camera ? camera : light;
                 int& size = w.camera ? camera_size : light_size;
                 const Vec<N, T> v = -w.ray.dir;
@@ -492,8 +498,19 @@ struct Bpt final
                 const Material<T, C>& m = s.materials[material];
                 const Vec<N, T>& n = normals.shading;
                 BrdfTerms terms;
-                const BrdfSample<N, C, T> bs =
-                        brdf_sample<N>(g, s.shading, m.roughness, m.f0, m.rho_ss, n, v, RECORD ? &terms : nullptr);
+                BrdfSample<N, C, T> bs;
+                if constexpr (N == 4 && sizeof(T) == 4)
+                {
+                        // inlined, the 4-space sample rounds differently, up to
+                        // 8e-4 of a pixel at a GGX peak; the call costs 0.4 ms of
+                        // 6.3 (7 M paths)
+                        bs = brdf_sample_call<N>(g, s.shading, m.roughness, m.f0, m.rho_ss, n, v,
+                                                 RECORD ? &terms : nullptr);
+                }
+                else
+                {
+                        bs = brdf_sample<N>(g, s.shading, m.roughness, m.f0, m.rho_ss, n, v, RECORD ? &terms : nullptr);
+                }
                 bool ok = bs.pdf > 0 && !bs.brdf.is_black();
                 T n_l = 0;
                 if (ok)
@@ -624,86 +641,99 @@ struct Bpt final
                 return v != 0 ? v : T(1);
         }
 
+        // Single precision keeps a connection's vertices in registers and
+        // inlines compute_pdf() at its four places in mis_weight() (4-space
+        // spectral box: connect kernel 7.7 -> 5.1 ms); double precision's
+        // registers do not hold them, and it reads them where they are (4-space
+        // job of 405,000 paths: 0.69 ms; copied and called 1.13, copied and
+        // inlined 0.93).
+        using HeldVertex = std::conditional_t<sizeof(T) == 4, const PathVertex<N, T, C>, const PathVertex<N, T, C>&>;
+
+        __device__ __forceinline__ T connected_pdf(const PathVertex<N, T, C>& prev, const PathVertex<N, T, C>& v,
+                                                   const PathVertex<N, T, C>& next) const
+        {
+                if constexpr (sizeof(T) == 4)
+                {
+                        return compute_pdf(prev, v, next);
+                }
+                else
+                {
+                        return compute_pdf_call(prev, v, next);
+                }
+        }
+
+        NBPT_CALL T compute_pdf_call(const PathVertex<N, T, C>& prev, const PathVertex<N, T, C>& v,
+                                     const PathVertex<N, T, C>& next) const
+        {
+                return compute_pdf(prev, v, next);
+        }
+
         // The light subpath is `lp` (light[] or the single resampled light
         // vertex of an s = 1 strategy).
-        NBPT_CALL T mis_weight(const PathVertex<N, T, C>* lp, const int s_count, const int t_count) const
+        __device__ __forceinline__ T mis_weight(const PathVertex<N, T, C>* lp, const int s_count, const int t_count) const
         {
                 if (s_count + t_count == 2)
                 {
                         return 1;
                 }
-                T lf[MAX_PATH_VERTICES];
-                T lr[MAX_PATH_VERTICES];
-                T cf[MAX_PATH_VERTICES];
-                T cr[MAX_PATH_VERTICES];
-                for (int i = 0; i < s_count; ++i)
-                {
-                        lf[i] = lp[i].pdf_fwd;
-                        lr[i] = lp[i].pdf_rev;
-                }
-                for (int i = 0; i < t_count; ++i)
-                {
-                        if (camera[i].type == static_cast<int>(VertexType::CAMERA))
-                        {
-                                cf[i] = -1;
-                                cr[i] = -1;
-                        }
-                        else
-                        {
-                                cf[i] = camera[i].pdf_fwd;
-                                cr[i] = camera[i].pdf_rev;
-                        }
-                }
-
-                // set_reversed (mis.cpp:107-146)
+                // The pdfs are the vertices' own but for those that the connection
+                // changes (set_reversed, mis.cpp:107-146): the reverse pdf of the
+                // last two vertices of either subpath.  Only the indices from 1 on
+                // of the camera subpath are read, whose vertices have pdfs.
+                T light_last = 0;
+                T light_before = 0;
+                T camera_last;
+                T camera_before = 0;
+                HeldVertex cv = camera[t_count - 1];
+                HeldVertex cv_before = camera[t_count - 2];
                 if (s_count == 0)
                 {
-                        cr[t_count - 1] = s.lights[camera[t_count - 1].light].pdf;
-                        cr[t_count - 2] = compute_light_pdf(camera[t_count - 1], camera[t_count - 2]);
+                        camera_last = s.lights[cv.light].pdf;
+                        camera_before = compute_light_pdf(cv, cv_before);
                 }
                 else
                 {
-                        lr[s_count - 1] = compute_pdf(camera[t_count - 2], camera[t_count - 1], lp[s_count - 1]);
+                        HeldVertex lv = lp[s_count - 1];
+                        light_last = connected_pdf(cv_before, cv, lv);
                         if (t_count > 2)
                         {
-                                cr[t_count - 2] = compute_pdf(lp[s_count - 1], camera[t_count - 1], camera[t_count - 2]);
+                                camera_before = connected_pdf(lv, cv, cv_before);
                         }
                         if (s_count == 1)
                         {
-                                cr[t_count - 1] = compute_light_pdf(lp[0], camera[t_count - 1]);
+                                camera_last = compute_light_pdf(lv, cv);
                         }
                         else
                         {
-                                lr[s_count - 2] = compute_pdf(camera[t_count - 1], lp[s_count - 1], lp[s_count - 2]);
-                                cr[t_count - 1] = compute_pdf(lp[s_count - 2], lp[s_count - 1], camera[t_count - 1]);
+                                HeldVertex lv_before = lp[s_count - 2];
+                                light_before = connected_pdf(cv, lv, lv_before);
+                                camera_last = connected_pdf(lv_before, lv, cv);
                         }
                 }
 
                 // every vertex of these scenes is connectible (no specular
                 // surfaces, no delta lights)
                 T light_sum = 0;
-                if (s_count > 0)
                 {
                         T ri = 1;
-                        for (int i = s_count - 1; i > 0; --i)
+                        for (int i = s_count - 1; i >= 0; --i)
                         {
-                                ri *= map(lr[i]) / map(lf[i]);
+                                const T reverse = i == s_count - 1 ? light_last
+                                                                   : (i == s_count - 2 ? light_before : lp[i].pdf_rev);
+                                ri *= map(reverse) / map(lp[i].pdf_fwd);
                                 light_sum += ri;
                         }
-                        ri *= map(lr[0]) / map(lf[0]);
-                        light_sum += ri;
                 }
                 T camera_sum = 0;
-                if (t_count > 1)
                 {
                         T ri = 1;
-                        for (int i = t_count - 1; i > 1; --i)
+                        for (int i = t_count - 1; i >= 1; --i)
                         {
-                                ri *= map(cr[i]) / map(cf[i]);
+                                const T reverse = i == t_count - 1 ? camera_last
+                                                                   : (i == t_count - 2 ? camera_before : camera[i].pdf_rev);
+                                ri *= map(reverse) / map(camera[i].pdf_fwd);
                                 camera_sum += ri;
                         }
-                        ri *= map(cr[1]) / map(cf[1]);
-                        camera_sum += ri;
                 }
                 return 1 / (1 + light_sum + camera_sum);
         }
@@ -726,10 +756,10 @@ struct Bpt final
         // known to be open: with Sight::MESH or Sight::WHOLE the slot is
         // written all the same, and taken back when the line turns out
         // blocked.  BLOCKED: no contribution.
-        NBPT_CALL Sight connect_light(const int t_count, const int li, const ArriveSample<N, T, C>& as,
+        __device__ __forceinline__ Sight connect_light(const int t_count, const int li, const ArriveSample<N, T, C>& as,
                                       Color<C>& out) const
         {
-                const PathVertex<N, T, C>& cv = camera[t_count - 1];
+                HeldVertex cv = camera[t_count - 1];
                 const Light<N, T, C>& l = s.lights[li];
                 PathVertex<N, T, C> lv;
                 lv.type = static_cast<int>(VertexType::LIGHT);
@@ -760,6 +790,9 @@ struct Bpt final
                 {
                         return sight;
                 }
+                lv.pos = opaque(lv.pos);
+                lv.dir = opaque(lv.dir);
+                lv.pdf_fwd = opaque(lv.pdf_fwd);
                 const float mis = static_cast<float>(mis_weight(&lv, 1, t_count));
                 out = c * mis;
                 if constexpr (RECORD)
@@ -776,9 +809,9 @@ struct Bpt final
                 return sight;
         }
 
-        NBPT_CALL Sight connect_strategy(const int s_count, const int t_count, Color<C>& out)
+        __device__ __forceinline__ Sight connect_strategy(const int s_count, const int t_count, Color<C>& out)
         {
-                const PathVertex<N, T, C>& cv = camera[t_count - 1];
+                HeldVertex cv = camera[t_count - 1];
                 if (s_count == 0)
                 {
                         if (cv.type != static_cast<int>(VertexType::SURFACE) || cv.light < 0)
@@ -822,7 +855,7 @@ struct Bpt final
                         return connect_light(t_count, li, as, out);
                 }
 
-                const PathVertex<N, T, C>& lv = light[s_count - 1];
+                HeldVertex lv = light[s_count - 1];
                 // compute_color (connect.cpp:187-221)
                 const Vec<N, T> v = lv.pos - cv.pos;
                 const T distance = v.norm();

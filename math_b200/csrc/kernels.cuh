@@ -378,7 +378,7 @@ __device__ inline unsigned reserve_together(unsigned* const counter, const unsig
 // The light sample of an s = 1 strategy (Bpt::light_arrival), kept for the
 // connect kernel.
 template <int N, typename T>
-struct Arrival final
+struct alignas(16) Arrival final
 {
         Vec<N, T> l;
         T pdf;

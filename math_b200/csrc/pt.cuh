@@ -140,9 +140,9 @@ struct Pt final
                 out.zero = (dot(n, v) <= 0 || dot(n, l) <= 0) ? 1 : 0;
                 if (!out.zero)
                 {
-                        out.terms = brdf_terms<N>(s.shading, m.roughness, n, v, l);
+                        out.terms = brdf_terms_call<N>(s.shading, m.roughness, n, v, l);
                 }
-                const T pdf = brdf_pdf(s.shading, m.roughness, n, v, l);
+                const T pdf = brdf_pdf_call<N>(s.shading, m.roughness, n, v, l);
                 const T weight = power_heuristic(sample.pdf, pdf);
                 out.scale = static_cast<float>(weight * n_l / sample.pdf);
                 out.light = k;
@@ -158,7 +158,7 @@ struct Pt final
                 const Vec<N, T>& n = normals.shading;
                 const Material<T, 1>& m = s.materials[q.material(surface)];
                 const BrdfSample<N, 1, T> sample =
-                        brdf_sample<N>(g, s.shading, m.roughness, m.f0, m.rho_ss, n, v, &out.terms);
+                        brdf_sample_call<N>(g, s.shading, m.roughness, m.f0, m.rho_ss, n, v, &out.terms);
                 if (!(sample.pdf > 0 && !sample.brdf.is_black()))
                 {
                         return false;
@@ -193,7 +193,7 @@ struct Pt final
                 const Vec<N, T>& n = normals.shading;
                 const Material<T, 1>& m = s.materials[q.material(surface)];
                 const BrdfSample<N, 1, T> sample =
-                        brdf_sample<N>(g, s.shading, m.roughness, m.f0, m.rho_ss, n, v, &out.terms);
+                        brdf_sample_call<N>(g, s.shading, m.roughness, m.f0, m.rho_ss, n, v, &out.terms);
                 if (!(sample.pdf > 0 && !sample.brdf.is_black()))
                 {
                         return false;

@@ -38,7 +38,7 @@ enum class NormalType : int
 };
 
 template <int N, typename T>
-struct FlatShape final
+struct alignas(16) FlatShape final
 {
         FlatParallelotope<N, T> shape;
         T lo[N];
@@ -48,7 +48,7 @@ struct FlatShape final
 };
 
 template <int N, typename T>
-struct SolidShape final
+struct alignas(16) SolidShape final
 {
         SolidParallelotope<N, T> shape;
         T lo[N];
@@ -57,7 +57,7 @@ struct SolidShape final
 };
 
 template <int N, typename T>
-struct Facet final
+struct alignas(16) Facet final
 {
         Simplex<N, T> simplex; // plane possibly reversed (facet.cpp:113-118)
         int material;
@@ -117,7 +117,7 @@ struct MeshShape final
 };
 
 template <typename T, int C>
-struct Material final
+struct alignas(16) Material final
 {
         T roughness;
         Color<C> f0;
@@ -131,7 +131,7 @@ enum class LightType : int
 };
 
 template <int N, typename T, int C>
-struct Light final
+struct alignas(16) Light final
 {
         int type;
         Vec<N, T> org;             // parallelotope origin or ball centre

@@ -402,13 +402,17 @@ struct BrdfTerms final
 };
 
 template <int N, typename T>
-NBPT_HD_CALL BrdfTerms brdf_terms(
+NBPT_HD BrdfTerms brdf_terms(
         const ShadingConstants<T>& sc,
-        const T roughness,
-        const Vec<N, T>& n,
-        const Vec<N, T>& v,
-        const Vec<N, T>& l)
+        const T roughness_in,
+        const Vec<N, T>& n_in,
+        const Vec<N, T>& v_in,
+        const Vec<N, T>& l_in)
 {
+        const T roughness = opaque(roughness_in);
+        const Vec<N, T> n = opaque(n_in);
+        const Vec<N, T> v = opaque(v_in);
+        const Vec<N, T> l = opaque(l_in);
         const Vec<N, T> h = (l + v).normalized();
         const T n_l = dot(n, l);
         const T h_l = dot(h, l);
@@ -475,7 +479,16 @@ NBPT_HD Color<C> brdf_color(const ShadingConstants<T>& sc, const BrdfTerms& t, c
         return r;
 }
 
-template <int N, int C, typename T>
+// brdf_terms() out of line: for kernels that evaluate it at several places
+// with few registers (pt.cuh).
+template <int N, typename T>
+NBPT_HD_CALL BrdfTerms brdf_terms_call(const ShadingConstants<T>& sc, const T roughness, const Vec<N, T>& n,
+                                       const Vec<N, T>& v, const Vec<N, T>& l)
+{
+        return brdf_terms<N>(sc, roughness, n, v, l);
+}
+
+template <int N, int C, bool CALL = false, typename T>
 NBPT_HD Color<C> brdf_f_unchecked(
         const ShadingConstants<T>& sc,
         const T roughness,
@@ -486,7 +499,7 @@ NBPT_HD Color<C> brdf_f_unchecked(
         const Vec<N, T>& l,
         BrdfTerms* const terms = nullptr)
 {
-        const BrdfTerms t = brdf_terms<N>(sc, roughness, n, v, l);
+        const BrdfTerms t = CALL ? brdf_terms_call<N>(sc, roughness, n, v, l) : brdf_terms<N>(sc, roughness, n, v, l);
         if (terms)
         {
                 *terms = t;
@@ -533,19 +546,23 @@ NBPT_HD T pdf_ggx_cosine(
 
 // brdf::pdf (brdf.h:173-194)
 template <int N, typename T>
-NBPT_HD_CALL T brdf_pdf(
+NBPT_HD T brdf_pdf(
         const ShadingConstants<T>& sc,
-        const T roughness,
-        const Vec<N, T>& n,
-        const Vec<N, T>& v,
-        const Vec<N, T>& l)
+        const T roughness_in,
+        const Vec<N, T>& n_in,
+        const Vec<N, T>& v_in,
+        const Vec<N, T>& l_in)
 {
+        const T roughness = opaque(roughness_in);
+        const Vec<N, T> n = opaque(n_in);
+        const Vec<N, T> v = opaque(v_in);
+        const Vec<N, T> l = opaque(l_in);
         if (dot(n, v) <= 0)
         {
                 return 0;
         }
         const T alpha = square(roughness);
-        return pdf_ggx_cosine(sc, alpha, n, v, l, (v + l).normalized());
+        return opaque(pdf_ggx_cosine(sc, alpha, n, v, l, (v + l).normalized()));
 }
 
 template <int N, int C, typename T>
@@ -558,17 +575,20 @@ struct BrdfSample final
 
 // brdf::sample_f (brdf.h:109-141, 196-238): a 50/50 mix of GGX
 // visible-normal and cosine sampling.
-template <int N, int C, typename T>
-NBPT_HD_CALL BrdfSample<N, C, T> brdf_sample(
+template <int N, int C, bool CALL = false, typename T>
+NBPT_HD BrdfSample<N, C, T> brdf_sample(
         Pcg& g,
         const ShadingConstants<T>& sc,
-        const T roughness,
+        const T roughness_in,
         const Color<C>& f0,
         const Color<C>& rho_ss,
-        const Vec<N, T>& n,
-        const Vec<N, T>& v,
+        const Vec<N, T>& n_in,
+        const Vec<N, T>& v_in,
         BrdfTerms* const terms = nullptr)
 {
+        const T roughness = opaque(roughness_in);
+        const Vec<N, T> n = opaque(n_in);
+        const Vec<N, T> v = opaque(v_in);
         BrdfSample<N, C, T> s;
         s.pdf = 0;
         if (dot(n, v) <= 0)
@@ -599,8 +619,8 @@ NBPT_HD_CALL BrdfSample<N, C, T> brdf_sample(
                 h = (v + l).normalized();
         }
         const T pdf = pdf_ggx_cosine(sc, alpha, n, v, l, h);
-        s.l = l;
-        s.pdf = pdf;
+        s.l = opaque(l);
+        s.pdf = opaque(pdf);
         if (pdf <= 0)
         {
                 s.pdf = 0;
@@ -611,7 +631,23 @@ NBPT_HD_CALL BrdfSample<N, C, T> brdf_sample(
                 s.brdf = Color<C>::filled(0);
                 return s;
         }
-        s.brdf = brdf_f_unchecked<N>(sc, roughness, f0, rho_ss, n, v, l, terms);
+        s.brdf = brdf_f_unchecked<N, C, CALL>(sc, roughness, f0, rho_ss, n, v, l, terms);
         return s;
+}
+
+// brdf_sample() and brdf_pdf() out of line, like brdf_terms_call().
+template <int N, int C, typename T>
+NBPT_HD_CALL BrdfSample<N, C, T> brdf_sample_call(Pcg& g, const ShadingConstants<T>& sc, const T roughness,
+                                                  const Color<C>& f0, const Color<C>& rho_ss, const Vec<N, T>& n,
+                                                  const Vec<N, T>& v, BrdfTerms* const terms)
+{
+        return brdf_sample<N, C, true>(g, sc, roughness, f0, rho_ss, n, v, terms);
+}
+
+template <int N, typename T>
+NBPT_HD_CALL T brdf_pdf_call(const ShadingConstants<T>& sc, const T roughness, const Vec<N, T>& n, const Vec<N, T>& v,
+                             const Vec<N, T>& l)
+{
+        return brdf_pdf<N>(sc, roughness, n, v, l);
 }
 } // namespace nbpt
