@@ -572,10 +572,10 @@ __global__ void __launch_bounds__(CONNECT_THREADS) connect_sight_kernel(
         constexpr unsigned GROUPS = CONNECT_THREADS / WIDE;
         using B = Bpt<N, T, 1, true>;
         using G = GroupQueries<N, T, 1>;
-        __shared__ WideStack<T> stacks[GROUPS];
+        extern __shared__ __align__(16) unsigned char stacks[];
         QueryCounters counters{0, 0, 0, 0};
         const SceneQueries<N, T, 1> q{scene, counters};
-        const G group{q, stacks[threadIdx.x / WIDE]};
+        const G group{q, WideStack<T>::of_group(stacks, scene.wide_stack, CONNECT_THREADS)};
         const unsigned mesh_count = sights.count[0];
         const unsigned count = mesh_count + sights.count[1];
         // the warp's groups loop together

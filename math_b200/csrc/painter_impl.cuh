@@ -166,6 +166,17 @@ public:
         }
 };
 
+// dynamic shared memory beyond 48 KB has to be asked for
+template <typename Kernel>
+void allow_shared(Kernel* const kernel, const std::size_t bytes)
+{
+        if (bytes > 48 * 1024)
+        {
+                NBPT_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               static_cast<int>(bytes)));
+        }
+}
+
 inline unsigned blocks_for(const long long n, const int threads)
 {
         return static_cast<unsigned>((n + threads - 1) / threads);
@@ -1029,6 +1040,7 @@ class SceneT final : public Scene
         DeviceArray<std::uint32_t> d_indices_;
         DeviceArray<WideChild<N, T>> d_wide_;
         DeviceArray<LeafFacet<N, T>> d_leaf_facets_;
+        int wide_stack_ = wide_stack_entries(0);
         DeviceArray<Facet<N, T>> d_facets_;
         DeviceArray<Vec<N, T>> d_normals_;
         DeviceArray<Material<T, C>> d_materials_;
@@ -1780,7 +1792,7 @@ public:
                 wide_index.allocate(node_total_);
                 DeviceArray<unsigned> counter;
                 // the roots are the first wide nodes
-                counter.upload(std::vector<unsigned>(1, static_cast<unsigned>(meshes_.size())));
+                counter.upload(std::vector<unsigned>{static_cast<unsigned>(meshes_.size()), 0});
                 for (std::size_t k = 0; k < meshes_.size(); ++k)
                 {
                         const MeshHost& m = meshes_[k];
@@ -1792,9 +1804,10 @@ public:
                                 counter.get(), wide_index.get() + m.node_offset);
                 }
                 NBPT_CUDA(cudaGetLastError());
-                unsigned count = 0;
-                counter.download(&count, 1);
-                d_wide_.allocate(static_cast<std::size_t>(count) * WIDE);
+                unsigned counts[2] = {};
+                counter.download(counts, 2);
+                wide_stack_ = wide_stack_entries(static_cast<int>(counts[1]));
+                d_wide_.allocate(static_cast<std::size_t>(counts[0]) * WIDE);
                 d_leaf_facets_.allocate(facet_total_);
                 for (const MeshHost& m : meshes_)
                 {
@@ -2125,6 +2138,7 @@ public:
                 device_.indices = d_indices_.get();
                 device_.wide = d_wide_.get();
                 device_.leaf_facets = d_leaf_facets_.get();
+                device_.wide_stack = wide_stack_;
                 device_.facets = d_facets_.get();
                 device_.normals = d_normals_.get();
                 device_.materials = d_materials_.get();
@@ -2181,6 +2195,7 @@ public:
                         device_1_.indices = device_.indices;
                         device_1_.wide = device_.wide;
                         device_1_.leaf_facets = device_.leaf_facets;
+                        device_1_.wide_stack = device_.wide_stack;
                         device_1_.facets = device_.facets;
                         device_1_.normals = device_.normals;
                         device_1_.materials = d_materials_1_.get();
@@ -2354,10 +2369,10 @@ __global__ void __launch_bounds__(TRACE_THREADS) trace_kernel(
         double* __restrict__ point)
 {
         using G = GroupQueries<N, T, C>;
-        __shared__ WideStack<T> stacks[TRACE_THREADS / WIDE];
+        extern __shared__ __align__(16) unsigned char stacks[];
         QueryCounters counters{0, 0, 0, 0};
         const SceneQueries<N, T, C> q{scene, counters};
-        const G group{q, stacks[threadIdx.x / WIDE]};
+        const G group{q, WideStack<T>::of_group(stacks, scene.wide_stack, TRACE_THREADS)};
         const long long i = (blockIdx.x * static_cast<long long>(TRACE_THREADS) + threadIdx.x) / WIDE;
         const bool active = i < count;
         Vec<N, T> o = Vec<N, T>::filled(0);
@@ -2402,6 +2417,16 @@ __global__ void __launch_bounds__(TRACE_THREADS) trace_kernel(
         {
                 point[i * N + k] = h ? static_cast<double>(h.point[k]) : 0.0;
         }
+}
+
+template <int N, typename T, int C>
+void launch_trace(const DeviceScene<N, T, C>& scene, const double* rays, const long long count, const int any, int* kind,
+                  int* index, double* t, double* point)
+{
+        const std::size_t shared = wide_stack_bytes<T>(scene.wide_stack, TRACE_THREADS);
+        allow_shared(trace_kernel<N, T, C>, shared);
+        trace_kernel<N, T, C><<<blocks_for(count * WIDE, TRACE_THREADS), TRACE_THREADS, shared>>>(
+                scene, rays, count, any, kind, index, t, point);
 }
 
 template <int N, typename T, int C>
@@ -3060,6 +3085,11 @@ public:
                         launches_accumulate_ = 0;
                         DeviceScene<N, T, 1> scene_1 = scene_->device_channel_0();
                         scene_1.flat_shading = flat_shading_ ? 1 : 0;
+                        if (integrator_ == Integrator::BPT)
+                        {
+                                allow_shared(walk_kernels().mesh, wide_stack_bytes<T>(scene_1.wide_stack, WALK_THREADS));
+                                allow_shared(sight_kernel(), wide_stack_bytes<T>(scene_1.wide_stack, CONNECT_THREADS));
+                        }
                         if (integrator_ == Integrator::PT)
                         {
                                 // one launch per chunk: whole paths (pt.cuh)
@@ -3127,7 +3157,9 @@ public:
                                         NBPT_CUDA(cudaGetLastError());
                                         if (scene_1.mesh_count > 0)
                                         {
-                                                sight_kernel()<<<walk_blocks_, 128, 0, stream_>>>(
+                                                sight_kernel()<<<walk_blocks_, CONNECT_THREADS,
+                                                                 wide_stack_bytes<T>(scene_1.wide_stack, CONNECT_THREADS),
+                                                                 stream_>>>(
                                                         scene_1, max_depth_, vertices_.get(), tape_.get(), tape_words_,
                                                         arrivals_.get(), sights, stats_.get());
                                                 NBPT_CUDA(cudaGetLastError());
@@ -3240,17 +3272,6 @@ public:
                 {
                         static_assert(C == 3);
                         accumulate_groups(screen, alpha, exp_radius, state);
-                }
-        }
-
-        // dynamic shared memory beyond 48 KB has to be asked for
-        template <typename Kernel>
-        static void allow_shared(Kernel* const kernel, const std::size_t bytes)
-        {
-                if (bytes > 48 * 1024)
-                {
-                        NBPT_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                       static_cast<int>(bytes)));
                 }
         }
 
@@ -3434,8 +3455,7 @@ void SceneT<N, T, C>::trace(
         d_t.allocate(count);
         DeviceArray<double> d_point;
         d_point.allocate(count * N);
-        trace_kernel<N, T, C><<<blocks_for(count * WIDE, TRACE_THREADS), TRACE_THREADS>>>(s, d_rays.get(), count, any, d_kind.get(), d_index.get(),
-                                                               d_t.get(), d_point.get());
+        launch_trace(s, d_rays.get(), count, any, d_kind.get(), d_index.get(), d_t.get(), d_point.get());
         NBPT_CUDA(cudaGetLastError());
         NBPT_CUDA(cudaDeviceSynchronize());
         d_kind.download(kind, count);
@@ -3458,7 +3478,7 @@ void SceneT<N, T, C>::trace_device(
         double* point) const
 {
         const DeviceScene<N, T, C>& s = device();
-        trace_kernel<N, T, C><<<blocks_for(count * WIDE, TRACE_THREADS), TRACE_THREADS>>>(s, rays, count, any, kind, index, t, point);
+        launch_trace(s, rays, count, any, kind, index, t, point);
         NBPT_CUDA(cudaGetLastError());
 }
 

@@ -197,6 +197,7 @@ struct DeviceScene final
         const std::uint32_t* indices;
         const WideChild<N, T>* wide; // the root of mesh m is wide node m
         const LeafFacet<N, T>* leaf_facets;
+        int wide_stack; // stack entries of a query (wide_stack_entries)
         const Facet<N, T>* facets;
         const Vec<N, T>* normals;
         const Material<T, C>* materials;

@@ -272,10 +272,10 @@ __global__ void __launch_bounds__(WALK_THREADS) walk_mesh_kernel(
 {
         constexpr unsigned GROUPS = WALK_THREADS / WIDE;
         using G = GroupQueries<N, T, 1>;
-        __shared__ WideStack<T> stacks[GROUPS];
+        extern __shared__ __align__(16) unsigned char stacks[];
         QueryCounters counters{0, 0, 0, 0};
         const SceneQueries<N, T, 1> q{scene, counters};
-        const G group{q, stacks[threadIdx.x / WIDE]};
+        const G group{q, WideStack<T>::of_group(stacks, scene.wide_stack, WALK_THREADS)};
         const unsigned count = *mesh_count;
         // the warp's groups loop together
         for (unsigned first = blockIdx.x * GROUPS + threadIdx.x / 32 * (32 / WIDE); first < count;
@@ -558,7 +558,7 @@ int launch_walks(const WalkKernels<N, T>& kernels, const WalkBuffers<N, T>& buff
         {
                 if (meshes)
                 {
-                        kernels.mesh<<<grid, WALK_THREADS, 0, stream>>>(scene, w.list, w.mesh_queue, w.mesh_count, stats);
+                        kernels.mesh<<<grid, WALK_THREADS, wide_stack_bytes<T>(scene.wide_stack, WALK_THREADS), stream>>>(scene, w.list, w.mesh_queue, w.mesh_count, stats);
                         ++launches;
                 }
         };

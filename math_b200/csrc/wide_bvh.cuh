@@ -17,8 +17,11 @@
 //     not depending on d; the binary traversal tests a box when it reaches
 //     it, so a stacked child keeps its near, which is compared with the
 //     distance of that moment.
-//   - Of a leaf's facets the closest one hit wins, the first of several at
-//     that distance, as when they are tested one by one.
+//   - Of a leaf's facets the closest one hit counts, the first of several at
+//     that distance, as when they are tested one by one; it is stacked with
+//     the leaf's near and wins if, when its turn comes, near does not exceed
+//     the distance and its own is smaller.  A facet that is not closer than
+//     the distance at the time of its test never will be.
 //
 // Why: rays that enter a mesh's box visit 79 binary nodes and 8 facets on
 // average on the 4-space hull of 20,000 points, 209 and 35 on a 5-space hull
@@ -36,9 +39,20 @@ inline constexpr int WIDE_LEVELS = 3;
 inline constexpr int WIDE = 1 << WIDE_LEVELS;
 inline constexpr std::uint32_t WIDE_LEAF = 1u << 31;
 
-// Entries of a ray's stack: a node leaves at most WIDE - 1 children behind
-// per level of wide nodes.
-inline constexpr int WIDE_STACK = ((host::BVH_MAX_DEPTH + WIDE_LEVELS - 1) / WIDE_LEVELS) * (WIDE - 1) + 1;
+// Entries of a ray's stack for trees of this depth: a node leaves at most
+// WIDE - 1 children behind per level of wide nodes.
+inline constexpr int wide_stack_entries(const int depth)
+{
+        const int levels = depth < 1 ? 1 : (depth + WIDE_LEVELS - 1) / WIDE_LEVELS;
+        return levels * (WIDE - 1) + 1;
+}
+
+// Dynamic shared memory of a block of `threads` threads.
+template <typename T>
+constexpr std::size_t wide_stack_bytes(const int entries, const int threads)
+{
+        return static_cast<std::size_t>(threads / WIDE) * entries * (2 * sizeof(T) + sizeof(std::uint32_t));
+}
 
 // ---------------------------------------------------------------------------
 // build, from the binary nodes of one mesh
@@ -68,7 +82,8 @@ __global__ void wide_parents_kernel(const BvhNode<N, T>* __restrict__ nodes, con
 template <int N, typename T>
 __global__ void wide_index_kernel(const BvhNode<N, T>* __restrict__ nodes, const int count,
                                   const std::uint32_t* __restrict__ parents, const std::uint32_t root,
-                                  unsigned* __restrict__ counter, std::uint32_t* __restrict__ wide_index)
+                                  unsigned* __restrict__ counter, // [2]: wide nodes, depth of the tree
+                                  std::uint32_t* __restrict__ wide_index)
 {
         const int i = static_cast<int>(blockIdx.x * blockDim.x + threadIdx.x);
         if (i >= count)
@@ -80,14 +95,19 @@ __global__ void wide_index_kernel(const BvhNode<N, T>* __restrict__ nodes, const
                 wide_index[0] = root;
                 return;
         }
-        if (nodes[i].count != 0)
-        {
-                return;
-        }
-        int depth = 0;
+        unsigned depth = 0;
         for (std::uint32_t p = parents[i]; p != ~0u; p = parents[p])
         {
                 ++depth;
+        }
+        if (nodes[i].count != 0)
+        {
+                // read first: few leaves deepen the tree
+                if (depth > *static_cast<volatile unsigned*>(counter + 1))
+                {
+                        atomicMax(counter + 1, depth);
+                }
+                return;
         }
         if (depth % WIDE_LEVELS == 0)
         {
@@ -176,12 +196,25 @@ __global__ void wide_facets_kernel(const Facet<N, T>* __restrict__ facets, const
 // queries: eight lanes per ray.  Every lane of the warp calls them, with its
 // group's ray; `active` and the results are equal in a group's lanes.
 
+// A group's stack, in dynamic shared memory.
 template <typename T>
 struct WideStack final
 {
-        T near[WIDE_STACK];
-        std::uint32_t ref[WIDE_STACK];
-        std::uint32_t facets[WIDE_STACK];
+        T* near;
+        T* distance;        // of a leaf's closest facet
+        std::uint32_t* ref; // wide node, or WIDE_LEAF | facet
+        int entries;
+
+        // the calling thread's group's, in wide_stack_bytes() of memory
+        __device__ static WideStack of_group(unsigned char* const memory, const int entries, const int threads)
+        {
+                const int groups = threads / WIDE;
+                const int group = static_cast<int>(threadIdx.x) / WIDE;
+                T* const near = reinterpret_cast<T*>(memory);
+                T* const distance = near + groups * entries;
+                std::uint32_t* const ref = reinterpret_cast<std::uint32_t*>(distance + groups * entries);
+                return {near + group * entries, distance + group * entries, ref + group * entries, entries};
+        }
 };
 
 template <int N, typename T, int C>
@@ -190,7 +223,7 @@ struct GroupQueries final
         static constexpr unsigned FULL = 0xffffffffu;
 
         const SceneQueries<N, T, C>& q;
-        WideStack<T>& stack; // the group's, in shared memory
+        const WideStack<T> stack;
 
         __device__ static unsigned lane()
         {
@@ -299,56 +332,56 @@ struct GroupQueries final
                         while (__any_sync(FULL, top > 0))
                         {
                                 bool node = false;
-                                bool leaf = false;
                                 std::uint32_t ref = 0;
-                                int facets = 0;
-                                while (top > 0 && !node && !leaf)
+                                while (top > 0 && !node)
                                 {
                                         --top;
-                                        if (stack.near[top] <= best)
+                                        if (!(stack.near[top] <= best))
                                         {
-                                                ref = stack.ref[top];
-                                                leaf = (ref & WIDE_LEAF) != 0;
-                                                node = !leaf;
-                                                facets = leaf ? static_cast<int>(stack.facets[top]) : 0;
+                                                continue;
+                                        }
+                                        ref = stack.ref[top];
+                                        node = (ref & WIDE_LEAF) == 0;
+                                        if (!ANY && !node && stack.distance[top] < best)
+                                        {
+                                                best = stack.distance[top];
+                                                kind = static_cast<int>(HitKind::FACET);
+                                                index = static_cast<int>(ref & ~WIDE_LEAF);
                                         }
                                 }
-                                __syncwarp(); // the entry is read before it is written again
-                                if (__any_sync(FULL, node))
-                                {
-                                        children(node, ref, ray, rec, neg, best, top);
-                                }
-                                if (__any_sync(FULL, leaf))
-                                {
-                                        leaf_facets<ANY>(facets, ref & ~WIDE_LEAF, ray, best, kind, index, top);
-                                }
+                                __syncwarp(); // the entries are read before they are written again
+                                children<ANY>(node, ref, ray, rec, neg, best, kind, top);
                         }
                 }
         }
 
 private:
-        // Tests the children of node `ref` and stacks those that are hit, the
-        // first to visit on top.
+        // Tests the children of node `ref`, and the facets of those that are
+        // leaves, and stacks what is hit, the first to visit on top.  ANY: a
+        // facet hit ends the query.
+        template <bool ANY>
         __device__ void children(const bool node, const std::uint32_t ref, const Ray<N, T>& ray, const Vec<N, T>& rec,
-                                 const unsigned neg, const T distance, int& top) const
+                                 const unsigned neg, const T best, int& kind, int& top) const
         {
                 using W = WideChild<N, T>;
                 bool hit = false;
                 T near = 0;
+                T closest = best;
+                std::uint32_t entry = 0;
                 unsigned key = 0;
-                W c;
+                int facets = 0; // of a leaf child that is hit
                 if (node)
                 {
-                        c = q.s.wide[static_cast<long long>(ref) * WIDE + lane()];
-                        T far = distance;
+                        const W c = q.s.wide[static_cast<long long>(ref) * WIDE + lane()];
+                        T far = best;
 #pragma unroll
                         for (int i = 0; i < N; ++i)
                         {
                                 const bool negative = (neg >> i) & 1u;
                                 const T a1 = ((negative ? c.hi[i] : c.lo[i]) - ray.org[i]) * rec[i];
                                 const T a2 = ((negative ? c.lo[i] : c.hi[i]) - ray.org[i]) * rec[i];
-                                near = a1 > near ? a1 : near;
-                                far = a2 < far ? a2 : far;
+                                near = slab_max(near, a1);
+                                far = slab_min(far, a2);
                         }
                         if (c.meta != W::UNUSED)
                         {
@@ -363,13 +396,29 @@ private:
                                 const unsigned axis = (c.meta >> W::axis_shift(level)) & W::NO_AXIS;
                                 key ^= ((neg >> axis) & 1u) << (WIDE_LEVELS - 1 - level);
                         }
+                        entry = c.ref;
+                        facets = hit && (c.ref & WIDE_LEAF) != 0 ? static_cast<int>(c.meta & W::COUNT_MASK) : 0;
+                }
+                if (__any_sync(FULL, facets > 0))
+                {
+                        leaf_facets<ANY>(facets, entry, ray, best, closest, hit);
+                }
+                if constexpr (ANY)
+                {
+                        const bool facet = hit && (entry & WIDE_LEAF) != 0;
+                        if (((__ballot_sync(FULL, facet) >> group_shift()) & 0xffu) != 0)
+                        {
+                                kind = static_cast<int>(HitKind::FACET);
+                                hit = false;
+                                top = 0;
+                        }
                 }
                 const unsigned hits =
                         (__reduce_or_sync(FULL, hit ? 1u << (group_shift() + key) : 0u) >> group_shift()) & 0xffu;
                 const int count = __popc(hits);
-                if (top + count > WIDE_STACK)
+                if (top + count > stack.entries)
                 {
-                        // the builders refuse trees this deep; end the query
+                        // the stacks are as deep as the trees; end the query
                         // rather than write past the stack
                         q.counters.overflows += lane() == 0 ? 1 : 0;
                         top = 0;
@@ -380,69 +429,123 @@ private:
                         {
                                 const int at = top + __popc(hits >> (key + 1));
                                 stack.near[at] = near;
-                                stack.ref[at] = c.ref;
-                                stack.facets[at] = c.meta & W::COUNT_MASK;
+                                stack.ref[at] = entry;
+                                if constexpr (!ANY)
+                                {
+                                        stack.distance[at] = closest;
+                                }
                         }
                         top += count;
                 }
                 __syncwarp();
         }
 
-        template <bool ANY>
-        __device__ void leaf_facets(const int count, const std::uint32_t slot, const Ray<N, T>& ray, T& best, int& kind,
-                                    int& index, int& top) const
+        __device__ T facet_distance(const std::uint32_t slot, const Ray<N, T>& ray, const T best, int& facet) const
         {
-                for (int first = 0; __any_sync(FULL, first < count); first += WIDE)
+                ++q.counters.facets;
+                const LeafFacet<N, T> f = q.s.leaf_facets[slot];
+                const T t = f.simplex.intersect_whole(ray);
+                facet = f.facet;
+                return t > 0 && t < best ? t : infinity<T>();
+        }
+
+        // The facets of the group's leaf children, `count` of this lane's
+        // from slot `entry` on (0: none); leaves `closest`, `entry` and `hit`
+        // as the lane would by testing its own one by one.  ANY: `hit` in some
+        // lane of the group when a facet is hit.
+        //
+        // Leaves hold 1 to 3 facets as a rule and few of a warp's 32 children
+        // are leaves that are hit.  Where a lane has several they are shared
+        // out, a facet to a lane: tested by their own lanes they took as many
+        // rounds of nearly empty warps as the largest leaf has facets (5-space
+        // job: mesh kernels 5.6 -> 4.8 ms).
+        template <bool ANY>
+        __device__ void leaf_facets(const int count, std::uint32_t& entry, const Ray<N, T>& ray, const T best, T& closest,
+                                    bool& hit) const
+        {
+                if (!__any_sync(FULL, count > 1))
                 {
-                        const int k = first + static_cast<int>(lane());
-                        T t = infinity<T>();
-                        int facet = -1;
-                        bool hit = false;
-                        if (k < count)
+                        if (count > 0)
                         {
-                                ++q.counters.facets;
-                                const LeafFacet<N, T> f = q.s.leaf_facets[static_cast<long long>(slot) + k];
-                                const T x = f.simplex.intersect_whole(ray);
-                                if (x > 0 && x < best)
-                                {
-                                        t = x;
-                                        facet = f.facet;
-                                        hit = true;
-                                }
+                                int facet;
+                                const T t = facet_distance(entry & ~WIDE_LEAF, ray, best, facet);
+                                hit = t < best;
+                                closest = hit ? t : closest;
+                                entry = WIDE_LEAF | static_cast<std::uint32_t>(facet);
                         }
-                        const unsigned hits = (__ballot_sync(FULL, hit) >> group_shift()) & 0xffu;
+                        return;
+                }
+                const int me = static_cast<int>(lane());
+                int end = count; // of the lane's facets among the group's
+#pragma unroll
+                for (int o = 1; o < WIDE; o <<= 1)
+                {
+                        const int x = __shfl_up_sync(FULL, end, o, WIDE);
+                        end += me >= o ? x : 0;
+                }
+                const int begin = end - count;
+                const int total = __shfl_sync(FULL, end, WIDE - 1, WIDE);
+                const std::uint32_t first_slot = (entry & ~WIDE_LEAF) - static_cast<std::uint32_t>(begin);
+                hit = hit && count == 0;
+                for (int first = 0; __any_sync(FULL, first < total); first += WIDE)
+                {
+                        const int j = first + me;
+                        int owner = 0;
+#pragma unroll
+                        for (int o = WIDE / 2; o > 0; o >>= 1)
+                        {
+                                owner += __shfl_sync(FULL, end, owner + o - 1, WIDE) <= j ? o : 0;
+                        }
+                        const std::uint32_t slot = __shfl_sync(FULL, first_slot, owner, WIDE);
+                        T t = infinity<T>();
+                        int facet = 0;
+                        if (j < total)
+                        {
+                                t = facet_distance(slot + static_cast<std::uint32_t>(j), ray, best, facet);
+                        }
                         if constexpr (ANY)
                         {
-                                if (hits != 0)
+                                if (t < best)
                                 {
-                                        kind = static_cast<int>(HitKind::FACET);
-                                        top = 0;
+                                        entry = WIDE_LEAF;
+                                        hit = true;
                                 }
                         }
                         else
                         {
-                                // the closest of the group's hits, the first of several
-                                int winner = 0;
-                                T closest = t;
-#pragma unroll
-                                for (int i = 0; i < WIDE; ++i)
+                                const int stop = min(end, first + WIDE);
+                                for (int k = max(begin, first); __any_sync(FULL, k < stop); ++k)
                                 {
-                                        const T x = __shfl_sync(FULL, t, i, WIDE);
-                                        if (i == 0 || x < closest)
+                                        const T x = __shfl_sync(FULL, t, k, WIDE);
+                                        const int f = __shfl_sync(FULL, facet, k, WIDE);
+                                        if (k < stop && x < closest)
                                         {
                                                 closest = x;
-                                                winner = i;
+                                                entry = WIDE_LEAF | static_cast<std::uint32_t>(f);
+                                                hit = true;
                                         }
-                                }
-                                const int f = __shfl_sync(FULL, facet, winner, WIDE);
-                                if (hits != 0)
-                                {
-                                        best = closest;
-                                        kind = static_cast<int>(HitKind::FACET);
-                                        index = f;
                                 }
                         }
                 }
+        }
+
+        // near and far of the slab test (box_hit): a NaN product, of a zero
+        // distance and an infinite reciprocal, changes neither
+        __device__ static float slab_max(const float near, const float a)
+        {
+                return fmaxf(near, a);
+        }
+        __device__ static double slab_max(const double near, const double a)
+        {
+                return a > near ? a : near;
+        }
+        __device__ static float slab_min(const float far, const float a)
+        {
+                return fminf(far, a);
+        }
+        __device__ static double slab_min(const double far, const double a)
+        {
+                return a < far ? a : far;
         }
 };
 } // namespace nbpt
