@@ -566,14 +566,14 @@ struct Bpt final
                 }
                 if constexpr (RECORD)
                 {
-                        tape.put(static_cast<int>(w.camera ? TapeRecord::CAMERA_BOUNCE : TapeRecord::LIGHT_BOUNCE));
-                        tape.put(material);
-                        tape.put(terms);
-                        tape.put(sample_k);
-                        if (!w.camera)
-                        {
-                                tape.put(normals_k);
-                        }
+                        static_assert(TAPE_CAMERA_BOUNCE == TAPE_LIGHT_BOUNCE);
+                        TapeWords<TAPE_LIGHT_BOUNCE> r;
+                        r.put(static_cast<int>(w.camera ? TapeRecord::CAMERA_BOUNCE : TapeRecord::LIGHT_BOUNCE));
+                        r.put(material);
+                        r.put(terms);
+                        r.put(sample_k);
+                        r.put(normals_k);
+                        tape.append(r);
                 }
                 if (w.beta.is_black() || ++w.depth == max_depth)
                 {
@@ -625,9 +625,11 @@ struct Bpt final
                 const float start_k = static_cast<float>(k / pdf);
                 if constexpr (RECORD)
                 {
-                        tape.put(static_cast<int>(TapeRecord::LIGHT_START));
-                        tape.put(li);
-                        tape.put(start_k);
+                        TapeWords<TAPE_LIGHT_START> r;
+                        r.put(static_cast<int>(TapeRecord::LIGHT_START));
+                        r.put(li);
+                        r.put(start_k);
+                        tape.append(r);
                 }
                 w = Walk{ls.radiance * start_k, ls.pdf_dir, ls.ray, 0, false};
                 return true;
@@ -797,14 +799,15 @@ struct Bpt final
                 out = c * mis;
                 if constexpr (RECORD)
                 {
-                        tape.n = tape_slot_offset(max_depth, t_count, 1);
-                        tape.put(static_cast<int>(TapeRecord::STRATEGY_LIGHT));
-                        tape.put(t_count);
-                        tape.put(cv.material);
-                        tape.put(terms);
-                        tape.put(li);
-                        tape.put(light_k);
-                        tape.put(mis);
+                        TapeWords<TAPE_STRATEGY_LIGHT> r;
+                        r.put(static_cast<int>(TapeRecord::STRATEGY_LIGHT));
+                        r.put(t_count);
+                        r.put(cv.material);
+                        r.put(terms);
+                        r.put(li);
+                        r.put(light_k);
+                        r.put(mis);
+                        tape.write(tape_slot_offset(max_depth, t_count, 1), r);
                 }
                 return sight;
         }
@@ -832,11 +835,12 @@ struct Bpt final
                         out = c * mis;
                         if constexpr (RECORD)
                         {
-                                tape.n = tape_slot_offset(max_depth, t_count, s_count);
-                                tape.put(static_cast<int>(TapeRecord::STRATEGY_EMITTED));
-                                tape.put(t_count);
-                                tape.put(cv.light);
-                                tape.put(mis);
+                                TapeWords<TAPE_STRATEGY_EMITTED> r;
+                                r.put(static_cast<int>(TapeRecord::STRATEGY_EMITTED));
+                                r.put(t_count);
+                                r.put(cv.light);
+                                r.put(mis);
+                                tape.write(tape_slot_offset(max_depth, t_count, s_count), r);
                         }
                         return Sight::OPEN;
                 }
@@ -891,16 +895,17 @@ struct Bpt final
                 out = c * mis;
                 if constexpr (RECORD)
                 {
-                        tape.n = tape_slot_offset(max_depth, t_count, s_count);
-                        tape.put(static_cast<int>(TapeRecord::STRATEGY_CONNECT));
-                        tape.put(s_count);
-                        tape.put(t_count);
-                        tape.put(cv.material);
-                        tape.put(camera_terms);
-                        tape.put(lv.material);
-                        tape.put(light_terms);
-                        tape.put(geometry_k);
-                        tape.put(mis);
+                        TapeWords<TAPE_STRATEGY_CONNECT> r;
+                        r.put(static_cast<int>(TapeRecord::STRATEGY_CONNECT));
+                        r.put(s_count);
+                        r.put(t_count);
+                        r.put(cv.material);
+                        r.put(camera_terms);
+                        r.put(lv.material);
+                        r.put(light_terms);
+                        r.put(geometry_k);
+                        r.put(mis);
+                        tape.write(tape_slot_offset(max_depth, t_count, s_count), r);
                 }
                 return sight;
         }

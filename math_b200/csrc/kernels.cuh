@@ -833,6 +833,7 @@ __global__ void __launch_bounds__(128) paths_replay_kernel(
         r.n = TAPE_HEADER;
         while (r.n < used)
         {
+                const int record = r.n;
                 const TapeRecord kind = static_cast<TapeRecord>(r.get_int());
                 if (kind == TapeRecord::CAMERA_BOUNCE)
                 {
@@ -847,6 +848,7 @@ __global__ void __launch_bounds__(128) paths_replay_kernel(
                                 camera_beta[camera_vertex + 1][k] = camera_beta[camera_vertex][k] * (b * sk);
                         }
                         ++camera_vertex;
+                        r.n = record + TAPE_CAMERA_BOUNCE;
                 }
                 else if (kind == TapeRecord::LIGHT_START)
                 {
@@ -858,6 +860,7 @@ __global__ void __launch_bounds__(128) paths_replay_kernel(
                                 light_beta[1][k] = l.radiance.c[lane + LANES * k] * sk;
                         }
                         light_vertex = 1;
+                        r.n = record + TAPE_LIGHT_START;
                 }
                 else if (kind == TapeRecord::LIGHT_BOUNCE)
                 {
@@ -874,6 +877,7 @@ __global__ void __launch_bounds__(128) paths_replay_kernel(
                                 light_beta[light_vertex + 1][k] = beta * nk;
                         }
                         ++light_vertex;
+                        r.n = record + TAPE_LIGHT_BOUNCE;
                 }
                 else
                 {

@@ -35,12 +35,18 @@ enum class TapeRecord : int
 // camera subpath size, light subpath size
 inline constexpr int TAPE_HEADER = 4;
 inline constexpr int TAPE_TERMS = 6;  // words of a BrdfTerms
-inline constexpr int TAPE_CAMERA_BOUNCE = 3 + TAPE_TERMS;
-inline constexpr int TAPE_LIGHT_START = 3;
-inline constexpr int TAPE_LIGHT_BOUNCE = 4 + TAPE_TERMS;
-inline constexpr int TAPE_STRATEGY_EMITTED = 4;
-inline constexpr int TAPE_STRATEGY_LIGHT = 6 + TAPE_TERMS;
-inline constexpr int TAPE_STRATEGY_CONNECT = 7 + 2 * TAPE_TERMS;
+// Records are multiples of four words, written and read 16 bytes at a time:
+// the lanes of a warp write to tapes of their own, a line each per write.
+inline constexpr int tape_record(const int words)
+{
+        return (words + 3) / 4 * 4;
+}
+inline constexpr int TAPE_CAMERA_BOUNCE = tape_record(3 + TAPE_TERMS);
+inline constexpr int TAPE_LIGHT_START = tape_record(3);
+inline constexpr int TAPE_LIGHT_BOUNCE = tape_record(4 + TAPE_TERMS);
+inline constexpr int TAPE_STRATEGY_EMITTED = tape_record(4);
+inline constexpr int TAPE_STRATEGY_LIGHT = tape_record(6 + TAPE_TERMS);
+inline constexpr int TAPE_STRATEGY_CONNECT = tape_record(7 + 2 * TAPE_TERMS);
 
 // Layout of one path's tape for a maximum depth D: the header; the bounce
 // records in the order they happen (at most D per subpath and the light
@@ -76,20 +82,31 @@ NBPT_HD constexpr int tape_words(const int max_depth)
 
 static_assert(tape_slot(6, 2, 6) == 6 && tape_slot(6, 3, 0) == 7 && tape_slot(6, 7, 1) == tape_slot_count(6) - 1);
 
-// Appends records to one path's tape (a contiguous slot of 32-bit words).
-struct TapeWriter final
+static_assert(tape_words(1) % 4 == 0 && tape_words(8) % 4 == 0);
+
+NBPT_HD std::uint32_t tape_bits(const float v)
 {
-        std::uint32_t* w = nullptr;
-        int n = TAPE_HEADER;
+        std::uint32_t u;
+        __builtin_memcpy(&u, &v, sizeof(u));
+        return u;
+}
+
+// A record of WORDS words, put together in registers.
+template <int WORDS>
+struct TapeWords final
+{
+        static constexpr int QUADS = tape_record(WORDS) / 4;
+        uint4 q[QUADS] = {};
+        int n = 0;
 
         NBPT_HD void put(const int v)
         {
-                w[n++] = static_cast<std::uint32_t>(v);
+                word(n++) = static_cast<std::uint32_t>(v);
         }
 
         NBPT_HD void put(const float v)
         {
-                w[n++] = bits_of(v);
+                word(n++) = tape_bits(v);
         }
 
         NBPT_HD void put(const BrdfTerms& t)
@@ -102,15 +119,43 @@ struct TapeWriter final
                 put(t.ggx_on);
         }
 
-        NBPT_HD static std::uint32_t bits_of(const float v)
+private:
+        NBPT_HD std::uint32_t& word(const int i)
         {
-                std::uint32_t u;
-                __builtin_memcpy(&u, &v, sizeof(u));
-                return u;
+                uint4& v = q[i / 4];
+                return i % 4 == 0 ? v.x : (i % 4 == 1 ? v.y : (i % 4 == 2 ? v.z : v.w));
         }
 };
 
-// Reads one path's tape.
+// One path's tape (a contiguous, 16-byte aligned slot of 32-bit words):
+// bounce records appended at `n`, strategy records at their slots.
+struct TapeWriter final
+{
+        std::uint32_t* w = nullptr;
+        int n = TAPE_HEADER;
+
+        template <int WORDS>
+        NBPT_HD void append(const TapeWords<WORDS>& r)
+        {
+                write(n, r);
+                n += tape_record(WORDS);
+        }
+
+        template <int WORDS>
+        NBPT_HD void write(const int at, const TapeWords<WORDS>& r) const
+        {
+                uint4* const to = reinterpret_cast<uint4*>(w + at);
+#pragma unroll
+                for (int i = 0; i < TapeWords<WORDS>::QUADS; ++i)
+                {
+                        to[i] = r.q[i];
+                }
+        }
+};
+
+// Reads one path's tape, word by word: the lanes of a warp read the same
+// words, and only those that a record has (whole records in 16-byte loads, a
+// run of paths per warp, were 10 % slower).
 struct TapeReader final
 {
         const std::uint32_t* w;
