@@ -79,7 +79,7 @@ struct ColorGroup final
 {
         const float* colors; // the source pixel's sample colours [spp][stride]
         const float* weights;
-        const float* contributions;
+        const float* lum; // the source pixel's sample luminances
         const int* order;
         int n;
         // channel c of this group is channel c * step + offset of the colours
@@ -95,6 +95,48 @@ struct ColorGroup final
                 return weights[i] * colors[i * stride + c * step + offset];
         }
 };
+
+// create_with_sum (samples/com/create.h:28-55): the sums of a group of more
+// than HELD_OUT samples, without those held out, in order.  Four samples'
+// colours are loaded before the first is added, since each is a load whose
+// address another load gives (64 channels, 27 groups of 27 samples per pixel:
+// with the merges as selections (FullMerge) 12.5 -> 10.3 ms for
+// 262,144 pixels).
+template <int C, typename S>
+__device__ void sum_group(const ColorGroup<C>& g, S (&sum)[C], S& wsum)
+{
+        constexpr int BATCH = 8;
+        const int last = g.n - HELD_OUT / 2;
+        for (int first = HELD_OUT / 2; first < last; first += BATCH)
+        {
+                float w[BATCH];
+                float c[BATCH][C];
+#pragma unroll
+                for (int b = 0; b < BATCH; ++b)
+                {
+                        const int i = g.order[min(first + b, last - 1)];
+                        w[b] = g.weights[i];
+#pragma unroll
+                        for (int k = 0; k < C; ++k)
+                        {
+                                c[b][k] = g.colors[i * g.stride + k * g.step + g.offset];
+                        }
+                }
+#pragma unroll
+                for (int b = 0; b < BATCH; ++b)
+                {
+                        if (first + b < last)
+                        {
+#pragma unroll
+                                for (int k = 0; k < C; ++k)
+                                {
+                                        sum[k] += w[b] * c[b][k];
+                                }
+                                wsum += w[b];
+                        }
+                }
+        }
+}
 
 // ---- merges (com/merge.h) ------------------------------------------------
 
@@ -131,7 +173,8 @@ struct SetView final
                 {
                         return s->contributions[k];
                 }
-                return g->contributions[g->order[group_position(k)]];
+                const int i = g->order[group_position(k)];
+                return g->weights[i] * g->lum[i];
         }
 
         NBPT_HD float weight(const int k) const
@@ -175,6 +218,51 @@ NBPT_HD void sum_entry(S* color_sum, S& weight_sum, const SetView<C, S>& from, c
         }
         weight_sum += from.weight(k);
 }
+
+// The choice merge_with_sum makes between two full sets, once for all their
+// values: of either half the two outermost of the four entries are held out
+// and the other two summed, a's before b's, the low half first.  Written out
+// as selections: with running indices the sets lay in local memory, a
+// dependent access per entry and channel.
+struct FullMerge final
+{
+        bool low_first; // a's entry is the first taken
+        bool low_second;
+        bool high_first;
+        bool high_second;
+
+        template <int C, typename S>
+        NBPT_HD FullMerge(const SetView<C, S>& a, const SetView<C, S>& b)
+        {
+                static_assert(HELD_OUT == 4);
+                low_first = a.contribution(0) < b.contribution(0);
+                low_second = low_first ? a.contribution(1) < b.contribution(0) : a.contribution(0) < b.contribution(1);
+                high_first = a.contribution(3) > b.contribution(3);
+                high_second = high_first ? a.contribution(2) > b.contribution(3) : a.contribution(3) > b.contribution(2);
+        }
+
+        // a(k), b(k): the values of the entries; out: those held out
+        template <typename A, typename B, typename S>
+        NBPT_HD void entries(const A& a, const B& b, float* const out, S& sum) const
+        {
+                const float a0 = a(0);
+                const float a1 = a(1);
+                const float a2 = a(2);
+                const float a3 = a(3);
+                const float b0 = b(0);
+                const float b1 = b(1);
+                const float b2 = b(2);
+                const float b3 = b(3);
+                out[0] = low_first ? a0 : b0;
+                out[1] = low_first ? (low_second ? a1 : b0) : (low_second ? a0 : b1);
+                out[3] = high_first ? a3 : b3;
+                out[2] = high_first ? (high_second ? a2 : b3) : (high_second ? a3 : b2);
+                sum += low_first && low_second ? b0 : (!low_first && !low_second ? a0 : a1);
+                sum += !low_first && !low_second ? a1 : b1;
+                sum += high_first && high_second ? b3 : (!high_first && !high_second ? a3 : a2);
+                sum += !high_first && !high_second ? a2 : b2;
+        }
+};
 
 // merge_with_sum (com/merge.h:199-233, samples/merge.cpp:109-145)
 template <int C, typename S>
@@ -227,48 +315,24 @@ NBPT_HD void merge_colors_with_sum(const SetView<C, S>& a, const SetView<C, S>& 
         ColorSet<C, S> r;
         if (a_size == HELD_OUT && b_size == HELD_OUT)
         {
-                int ai = 0;
-                int bi = 0;
-                for (int i = 0; i < HELD_OUT / 2; ++i)
+                const FullMerge m(a, b);
+#pragma unroll 8
+                for (int c = 0; c < C; ++c)
                 {
-                        if (a.contribution(ai) < b.contribution(bi))
+                        float out_c[HELD_OUT];
+                        m.entries([&](const int k) { return a.color(k, c); }, [&](const int k) { return b.color(k, c); },
+                                  out_c, sum[c]);
+#pragma unroll
+                        for (int k = 0; k < HELD_OUT; ++k)
                         {
-                                copy_entry(r, i, a, ai++);
-                        }
-                        else
-                        {
-                                copy_entry(r, i, b, bi++);
-                        }
-                }
-                while (ai < HELD_OUT / 2)
-                {
-                        sum_entry(sum, wsum, a, ai++);
-                }
-                while (bi < HELD_OUT / 2)
-                {
-                        sum_entry(sum, wsum, b, bi++);
-                }
-                ai = HELD_OUT - 1;
-                bi = HELD_OUT - 1;
-                for (int i = HELD_OUT - 1; i >= HELD_OUT / 2; --i)
-                {
-                        if (a.contribution(ai) > b.contribution(bi))
-                        {
-                                copy_entry(r, i, a, ai--);
-                        }
-                        else
-                        {
-                                copy_entry(r, i, b, bi--);
+                                r.colors[k][c] = out_c[k];
                         }
                 }
-                while (ai >= HELD_OUT / 2)
-                {
-                        sum_entry(sum, wsum, a, ai--);
-                }
-                while (bi >= HELD_OUT / 2)
-                {
-                        sum_entry(sum, wsum, b, bi--);
-                }
+                m.entries([&](const int k) { return a.weight(k); }, [&](const int k) { return b.weight(k); }, r.weights,
+                          wsum);
+                S unused = 0;
+                m.entries([&](const int k) { return a.contribution(k); }, [&](const int k) { return b.contribution(k); },
+                          r.contributions, unused);
         }
         else
         {
@@ -1092,7 +1156,6 @@ __global__ void __launch_bounds__(128) accumulate_warp_kernel(
         constexpr int K = C / 32;
         constexpr int WARPS = 4;
         __shared__ float s_weight[WARPS][MAX_GROUP];
-        __shared__ float s_contribution[WARPS][MAX_GROUP];
         __shared__ int s_kind[WARPS][MAX_GROUP]; // 0 none, 1 colour, 2 background
         __shared__ int s_order[WARPS][MAX_GROUP];
         __shared__ float s_background[WARPS][MAX_GROUP];
@@ -1107,7 +1170,6 @@ __global__ void __launch_bounds__(128) accumulate_warp_kernel(
                 return; // the whole warp
         }
         float* const w = s_weight[warp];
-        float* const contribution = s_contribution[warp];
         int* const kind = s_kind[warp];
         int* const order = s_order[warp];
         float* const background = s_background[warp];
@@ -1194,15 +1256,7 @@ __global__ void __launch_bounds__(128) accumulate_warp_kernel(
                         {
                                 const float wf = static_cast<float>(weight);
                                 w[j] = wf;
-                                if (valid[sidx])
-                                {
-                                        contribution[j] = wf * lum[sidx];
-                                        k = 1;
-                                }
-                                else
-                                {
-                                        k = 2;
-                                }
+                                k = valid[sidx] ? 1 : 2;
                         }
                         kind[j] = k;
                 }
@@ -1222,7 +1276,8 @@ __global__ void __launch_bounds__(128) accumulate_warp_kernel(
                                         background[nbg++] = w[j];
                                 }
                         }
-                        order_group(order, nc, [&](const int i) { return contribution[i]; });
+                        const float* const source_lum = lum + (p - screen.source_first) * spp;
+                        order_group(order, nc, [&](const int i) { return w[i] * source_lum[i]; });
                         if (nbg > 1)
                         {
                                 // background samples are ordered by value; reuse
@@ -1250,7 +1305,8 @@ __global__ void __launch_bounds__(128) accumulate_warp_kernel(
                 const int nbg = s_counts[warp][1];
                 if (nc > 0)
                 {
-                        const ColorGroup<K> g{colors + (p - screen.source_first) * spp * C, w, contribution, order, nc, C, 32, lane};
+                        const float* const source_lum = lum + (p - screen.source_first) * spp;
+                        const ColorGroup<K> g{colors + (p - screen.source_first) * spp * C, w, source_lum, order, nc, C, 32, lane};
                         S g_sum[K];
                         S g_wsum = 0;
 #pragma unroll
@@ -1261,15 +1317,7 @@ __global__ void __launch_bounds__(128) accumulate_warp_kernel(
                         const bool g_full = nc > HELD_OUT;
                         if (g_full)
                         {
-                                for (int k = HELD_OUT / 2; k < nc - HELD_OUT / 2; ++k)
-                                {
-#pragma unroll
-                                        for (int c = 0; c < K; ++c)
-                                        {
-                                                g_sum[c] += g.color(k, c);
-                                        }
-                                        g_wsum += w[order[k]];
-                                }
+                                sum_group(g, g_sum, g_wsum);
                         }
                         merge_color_group(cs, g, g_sum, g_wsum, g_full);
                 }
@@ -1331,7 +1379,6 @@ __global__ void __launch_bounds__(128) accumulate_warp_small_kernel(
         static_assert(N <= 4, "the shared-memory tables hold 3^(N-1) <= 27 neighbours");
         constexpr int NB = N == 3 ? 9 : 27;
         __shared__ float s_weight[WARPS][NB][SMALL_GROUP];
-        __shared__ float s_contribution[WARPS][NB][SMALL_GROUP];
         __shared__ unsigned char s_kind[WARPS][NB][SMALL_GROUP]; // 0 none, 1 colour, 2 background
         __shared__ unsigned char s_order[WARPS][NB][SMALL_GROUP];
         __shared__ unsigned char s_order_bg[WARPS][NB][SMALL_GROUP];
@@ -1406,15 +1453,7 @@ __global__ void __launch_bounds__(128) accumulate_warp_small_kernel(
                 {
                         const float wf = static_cast<float>(weight);
                         s_weight[warp][nb][j] = wf;
-                        if (valid[sidx])
-                        {
-                                s_contribution[warp][nb][j] = wf * lum[sidx];
-                                k = 1;
-                        }
-                        else
-                        {
-                                k = 2;
-                        }
+                        k = valid[sidx] ? 1 : 2;
                 }
                 s_kind[warp][nb][j] = k;
         }
@@ -1445,9 +1484,9 @@ __global__ void __launch_bounds__(128) accumulate_warp_small_kernel(
                                         order_bg[nbg++] = j;
                                 }
                         }
-                        const float* const contribution = s_contribution[warp][nb];
+                        const float* const source_lum = lum + (p - screen.source_first) * spp;
                         const float* const w = s_weight[warp][nb];
-                        order_group(order, nc, [&](const int i) { return contribution[i]; });
+                        order_group(order, nc, [&](const int i) { return w[i] * source_lum[i]; });
                         order_group(order_bg, nbg, [&](const int i) { return w[i]; });
                         for (int k = 0; k < nc; ++k)
                         {
@@ -1511,7 +1550,8 @@ __global__ void __launch_bounds__(128) accumulate_warp_small_kernel(
                 __syncwarp();
                 if (nc > 0)
                 {
-                        const ColorGroup<K> g{colors + (p - screen.source_first) * spp * C, w, s_contribution[warp][nb], order, nc, C, 32, lane};
+                        const float* const source_lum = lum + (p - screen.source_first) * spp;
+                        const ColorGroup<K> g{colors + (p - screen.source_first) * spp * C, w, source_lum, order, nc, C, 32, lane};
                         S g_sum[K];
                         S g_wsum = 0;
 #pragma unroll
@@ -1522,15 +1562,7 @@ __global__ void __launch_bounds__(128) accumulate_warp_small_kernel(
                         const bool g_full = nc > HELD_OUT;
                         if (g_full)
                         {
-                                for (int k = HELD_OUT / 2; k < nc - HELD_OUT / 2; ++k)
-                                {
-#pragma unroll
-                                        for (int c = 0; c < K; ++c)
-                                        {
-                                                g_sum[c] += g.color(k, c);
-                                        }
-                                        g_wsum += w[order[k]];
-                                }
+                                sum_group(g, g_sum, g_wsum);
                         }
                         merge_color_group(cs, g, g_sum, g_wsum, g_full);
                 }
