@@ -13,6 +13,7 @@
 #include "scene.cuh"
 #include "shading.cuh"
 #include "tape.cuh"
+#include "wide_bvh.cuh"
 
 #include <type_traits>
 
@@ -291,85 +292,47 @@ struct Bpt final
                 return cosine > EPSILON;
         }
 
-        NBPT_CALL bool move_and_intersect_any(const Vec<N, T>& gn, const Ray<N, T>& ray, const T distance) const
+        // occluded(scene, normals, ray, distance) (visibility.h:99-123) of a ray
+        // per lane; the warp calls it together
+        __device__ bool occluded_ray(const WarpQueries<N, T, C>& warp, const bool active, const Normals<N, T>& normals,
+                                     const Ray<N, T>& from, const T distance) const
         {
-                const Hit<N, T> h = q.intersect(&gn, ray, distance);
-                if (!h)
+                bool open = active;
+                bool moves = false;
+                Ray<N, T> ray = from;
+                T d = visibility_distance(distance);
+                if (active)
                 {
-                        return false;
+                        open = directed_outside(dot(from.dir, normals.shading));
+                        moves = open && !(dot(from.dir, normals.geometric) >= 0);
+                        ray.org = offset_ray_org(normals.geometric, from);
                 }
-                const T d = distance - h.distance;
-                if (d > 0)
+                const bool occluded = active && !open;
+                bool ask = open;
+                if (__any_sync(WarpQueries<N, T, C>::FULL, moves))
                 {
-                        const Vec<N, T> hg = q.geometric_normal(h);
-                        Ray<N, T> r2 = ray;
-                        r2.org = h.point;
-                        return q.intersect_any(&hg, r2, d);
-                }
-                return false;
-        }
-
-        // occluded(scene, normals, ray, distance) (visibility.h:99-123)
-        NBPT_CALL bool occluded_ray(const Normals<N, T>& normals, const Ray<N, T>& ray, const T distance) const
-        {
-                if (!directed_outside(dot(ray.dir, normals.shading)))
-                {
-                        return true;
-                }
-                const T d = visibility_distance(distance);
-                const bool visible = dot(ray.dir, normals.geometric) >= 0;
-                if (visible)
-                {
-                        return q.intersect_any(&normals.geometric, ray, d);
-                }
-                return move_and_intersect_any(normals.geometric, ray, d);
-        }
-
-        // occluded(scene, p1, n1, p2, n2) (visibility.h:125-172)
-        NBPT_CALL bool occluded_points(const Vec<N, T>& p1, const Normals<N, T>& n1, const Vec<N, T>& p2,
-                                        const Normals<N, T>& n2) const
-        {
-                const Vec<N, T> direction_1 = p2 - p1;
-                const Ray<N, T> ray_1 = Ray<N, T>::make(p1, direction_1);
-                if (!directed_outside(dot(ray_1.dir, n1.shading)) || !directed_outside(-dot(ray_1.dir, n2.shading)))
-                {
-                        return true;
-                }
-                const bool visible_1 = dot(ray_1.dir, n1.geometric) >= 0;
-                const bool visible_2 = dot(ray_1.dir, n2.geometric) <= 0;
-                T distance = visibility_distance(direction_1.norm());
-                if (visible_1 && visible_2)
-                {
-                        return q.intersect_any(&n1.geometric, ray_1, distance);
-                }
-                if (!visible_1)
-                {
-                        const Hit<N, T> h = q.intersect(&n1.geometric, ray_1, distance);
-                        if (!h)
+                        // the surface's other side first (move_and_intersect_any,
+                        // visibility.h)
+                        const Hit<N, T> h = warp.closest(moves, ray, d);
+                        if (moves)
                         {
-                                return false;
+                                ask = h && d - h.distance > 0;
+                                if (ask)
+                                {
+                                        d = d - h.distance;
+                                        ray.org = h.point;
+                                        ray.org = offset_ray_org(q.geometric_normal(h), ray);
+                                }
                         }
-                        const T d = distance - h.distance;
-                        if (!(d > 0))
-                        {
-                                return false;
-                        }
-                        distance = d;
                 }
-                Ray<N, T> ray_2;
-                ray_2.org = p2;
-                ray_2.dir = -ray_1.dir;
-                if (!visible_2)
-                {
-                        return move_and_intersect_any(n2.geometric, ray_2, distance);
-                }
-                return q.intersect_any(&n2.geometric, ray_2, distance);
+                return warp.any(ask, ray, d) || occluded;
         }
 
         // What a connection's thread finds out about its line of sight: the
         // flat and solid shapes decide, or the meshes must be asked (a ray
         // that may enter one), or the geometric and shading normals disagree
-        // and the whole of occluded_ray() / occluded_points() is needed.
+        // and the whole of the reference's occluded() is needed, with its queries
+        // for the surfaces' other sides.
         // The last two are answered by connect_sight_kernel.
         enum class Sight : int
         {
@@ -379,7 +342,7 @@ struct Bpt final
                 WHOLE = 3
         };
 
-        // the ray of intersect_any() against the shapes
+        // the any-hit ray against the shapes
         __device__ Sight shape_sight(const Vec<N, T>& normal, const Ray<N, T>& from, const T distance) const
         {
                 Ray<N, T> ray = from;
@@ -392,7 +355,7 @@ struct Bpt final
                 return q.enters_mesh(ray, distance) ? Sight::MESH : Sight::OPEN;
         }
 
-        // occluded_ray()
+        // occluded(scene, normals, ray, distance) (visibility.h:99-123)
         __device__ Sight ray_sight(const Normals<N, T>& normals, const Ray<N, T>& ray, const T distance) const
         {
                 if (!directed_outside(dot(ray.dir, normals.shading)))
@@ -407,7 +370,7 @@ struct Bpt final
                 return Sight::WHOLE;
         }
 
-        // occluded_points()
+        // occluded(scene, p1, n1, p2, n2) (visibility.h:125-172)
         __device__ Sight point_sight(const Vec<N, T>& p1, const Normals<N, T>& n1, const Vec<N, T>& p2,
                                      const Normals<N, T>& n2) const
         {

@@ -527,8 +527,8 @@ __global__ void __launch_bounds__(CONNECT_THREADS) paths_connect_kernel(
         add_counters(counters, stats);
 }
 
-// SceneQueries::intersect() for the groups that are `active`; the others'
-// `hit` stays.
+// A closest-hit query of the groups that are `active`; the others' `hit`
+// stays.
 template <int N, typename T>
 __device__ inline void group_closest(const GroupQueries<N, T, 1>& group, const bool active, const Vec<N, T>& normal,
                                      const Ray<N, T>& from, const T max_distance, Hit<N, T>& hit)
@@ -589,7 +589,7 @@ __global__ void __launch_bounds__(CONNECT_THREADS) connect_sight_kernel(
                 Ray<N, T> ray;
                 T distance = 0;
                 Vec<N, T> normal;
-                // WHOLE: the queries before the last one (occluded_points())
+                // WHOLE: the queries before the last one (visibility.h:125-172)
                 bool first_query = false;
                 bool second_query = false;
                 Ray<N, T> second;
@@ -632,7 +632,7 @@ __global__ void __launch_bounds__(CONNECT_THREADS) connect_sight_kernel(
                 bool open = !active; // decided
                 if (__any_sync(G::FULL, whole))
                 {
-                        // occluded_points(): the first query and the ray back
+                        // the first query and the ray back
                         Hit<N, T> hit;
                         group_closest(group, first_query, normal, ray, distance, hit);
                         if (first_query)

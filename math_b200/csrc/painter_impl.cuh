@@ -2858,9 +2858,14 @@ public:
                 if (integrator_ == Integrator::PT)
                 {
                         next_path_.allocate(1);
-                        connect_blocks_ = sms * NBPT_PT_MIN_BLOCKS;
+                        // as many blocks as the device holds at once
+                        const std::size_t shared = wide_stack_bytes<T>(scene_->device().wide_stack, PT_THREADS);
+                        allow_shared(pt_kernel(), shared);
+                        int resident = 0;
+                        NBPT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, pt_kernel(), PT_THREADS, shared));
+                        connect_blocks_ = sms * std::max(1, resident);
                         // direct-lighting records: 2 per light per thread
-                        pt_estimates_.allocate(std::max(1LL, static_cast<long long>(connect_blocks_) * 128 * 2 *
+                        pt_estimates_.allocate(std::max(1LL, static_cast<long long>(connect_blocks_) * PT_THREADS * 2 *
                                                                      scene_->device().light_count));
                 }
                 else
@@ -3100,7 +3105,8 @@ public:
                                         const long long n = (e - b) * spp_;
                                         NBPT_CUDA(cudaMemsetAsync(next_path_.get(), 0, sizeof(unsigned), stream_));
                                         pt_kernel()
-                                                <<<std::min<long long>(connect_blocks_, blocks_for(n, 128)), 128, 0, stream_>>>(
+                                                <<<std::min<long long>(connect_blocks_, blocks_for(n, PT_THREADS)), PT_THREADS,
+                                                   wide_stack_bytes<T>(scene_1.wide_stack, PT_THREADS), stream_>>>(
                                                         scene_1, scene_->device_materials(),
                                                         scene_->device_lights(), b, e, spp_, seed_, pass,
                                                         points_.get() + o * spp_ * (N - 1), colors_.get() + o * spp_ * C,

@@ -114,35 +114,41 @@ struct Pt final
         }
 
         // sample_light_with_mis (direct_lighting.cpp:59-99); the lights here
-        // are area lights (is_delta() false)
-        NBPT_CALL bool light_with_mis(const int k, const Hit<N, T>& surface, const Vec<N, T>& v,
-                                      const Normals<N, T>& normals, PtEstimate& out) const
+        // are area lights (is_delta() false).  The warp calls it together.
+        __device__ bool light_with_mis(const WarpQueries<N, T, 1>& warp, const bool active, const int k,
+                                       const Hit<N, T>& surface, const Vec<N, T>& v, const Normals<N, T>& normals,
+                                       PtEstimate& out) const
         {
                 const Light<N, T, 1>& light = s.lights[k];
                 const Vec<N, T>& n = normals.shading;
-                const ArriveSample<N, T, 1> sample = b.arrive_sample(light, surface.point);
-                if (!sample.usable())
+                ArriveSample<N, T, 1> sample;
+                bool ok = false;
+                T n_l = 0;
+                Ray<N, T> ray;
+                if (active)
+                {
+                        sample = b.arrive_sample(light, surface.point);
+                        ok = sample.usable();
+                        if (ok)
+                        {
+                                n_l = dot(n, sample.l);
+                                ok = n_l > 0;
+                                ray = Ray<N, T>::make(surface.point, sample.l);
+                        }
+                }
+                if (b.occluded_ray(warp, ok, normals, ray, sample.distance) || !ok)
                 {
                         return false;
                 }
                 const Vec<N, T>& l = sample.l;
-                const T n_l = dot(n, l);
-                if (!(n_l > 0))
-                {
-                        return false;
-                }
-                if (b.occluded_ray(normals, Ray<N, T>::make(surface.point, l), sample.distance))
-                {
-                        return false;
-                }
                 const Material<T, 1>& m = s.materials[q.material(surface)];
                 // brdf::f's own checks (brdf.h:146-171), then its terms
                 out.zero = (dot(n, v) <= 0 || dot(n, l) <= 0) ? 1 : 0;
                 if (!out.zero)
                 {
-                        out.terms = brdf_terms_call<N>(s.shading, m.roughness, n, v, l);
+                        out.terms = brdf_terms<N>(s.shading, m.roughness, n, v, l);
                 }
-                const T pdf = brdf_pdf_call<N>(s.shading, m.roughness, n, v, l);
+                const T pdf = brdf_pdf<N>(s.shading, m.roughness, n, v, l);
                 const T weight = power_heuristic(sample.pdf, pdf);
                 out.scale = static_cast<float>(weight * n_l / sample.pdf);
                 out.light = k;
@@ -150,32 +156,32 @@ struct Pt final
         }
 
         // sample_surface_with_mis (direct_lighting.cpp:101-147); no shape
-        // here is specular
-        NBPT_CALL bool surface_with_mis(const int k, const Hit<N, T>& surface, const Vec<N, T>& v,
-                                        const Normals<N, T>& normals, PtEstimate& out) const
+        // here is specular.  The warp calls it together.
+        __device__ bool surface_with_mis(const WarpQueries<N, T, 1>& warp, const bool active, const int k,
+                                         const Hit<N, T>& surface, const Vec<N, T>& v, const Normals<N, T>& normals,
+                                         PtEstimate& out) const
         {
                 const Light<N, T, 1>& light = s.lights[k];
                 const Vec<N, T>& n = normals.shading;
-                const Material<T, 1>& m = s.materials[q.material(surface)];
-                const BrdfSample<N, 1, T> sample =
-                        brdf_sample_call<N>(g, s.shading, m.roughness, m.f0, m.rho_ss, n, v, &out.terms);
-                if (!(sample.pdf > 0 && !sample.brdf.is_black()))
+                BrdfSample<N, 1, T> sample;
+                bool ok = false;
+                T n_l = 0;
+                T light_pdf = 0;
+                T distance = 0;
+                Ray<N, T> ray;
+                if (active)
                 {
-                        return false;
+                        const Material<T, 1>& m = s.materials[q.material(surface)];
+                        sample = brdf_sample_call<N>(g, s.shading, m.roughness, m.f0, m.rho_ss, n, v, &out.terms);
+                        ok = sample.pdf > 0 && !sample.brdf.is_black();
+                        if (ok)
+                        {
+                                n_l = dot(n, sample.l);
+                                ok = n_l > 0 && arrive_info(light, surface.point, sample.l, light_pdf, distance);
+                                ray = Ray<N, T>::make(surface.point, sample.l);
+                        }
                 }
-                const Vec<N, T>& l = sample.l;
-                const T n_l = dot(n, l);
-                if (!(n_l > 0))
-                {
-                        return false;
-                }
-                T light_pdf;
-                T distance;
-                if (!arrive_info(light, surface.point, l, light_pdf, distance))
-                {
-                        return false;
-                }
-                if (b.occluded_ray(normals, Ray<N, T>::make(surface.point, l), distance))
+                if (b.occluded_ray(warp, ok, normals, ray, distance) || !ok)
                 {
                         return false;
                 }
@@ -187,7 +193,7 @@ struct Pt final
         }
 
         // com::surface_sample (surface_sample.cpp:31-70)
-        NBPT_CALL bool continuation(const Hit<N, T>& surface, const Vec<N, T>& v, const Normals<N, T>& normals,
+        __device__ bool continuation(const Hit<N, T>& surface, const Vec<N, T>& v, const Normals<N, T>& normals,
                                     PtContinuation<N, T>& out) const
         {
                 const Vec<N, T>& n = normals.shading;
@@ -220,16 +226,21 @@ __device__ float pt_brdf_channel(const BrdfTerms& t, const int zero, const Mater
         return zero ? 0.0f : brdf_channel(t, m.f0.c[c], m.rho_ss.c[c], sc.fresnel_a, sc.fresnel_b);
 }
 
-#ifndef NBPT_PT_MIN_BLOCKS
-#define NBPT_PT_MIN_BLOCKS 16
-#endif
-
 // The PT integrator's paths (pt.cpp:113-170), one lane per path at a time
 // and one bounce per iteration of a persistent loop: every lane traces one
 // ray and processes its hit in each iteration, and a lane whose path ends
 // writes it out and takes the next path from a shared counter, so the
 // warp's lanes run together however many bounces Russian roulette gives
-// their paths.  The sample points, the path's ray and its random stream are
+// their paths.  The warp goes through a bounce as one: at every ray query its
+// lanes wait for each other and hand the rays that may enter a mesh to the
+// warp's groups of eight (WarpQueries), and the block's warps meet at barriers
+// between the parts of a bounce, so that they fetch the same instructions.
+// Left to themselves the lanes were at different parts of their bounces, 4 of
+// 32 active, with 64 warps per SM at 32 registers to hide it (3-space f64, two
+// passes of 1 M paths: 14.6 ms); warps in step each for itself are bound by
+// instruction fetch (21.8 ms), blocks of 256 or 512 threads in step are not
+// (9.3 ms; 4-space spectral f32, 3 M paths: 20.9 -> 17.0 ms, 22.6 with 512).
+// The sample points, the path's ray and its random stream are
 // those of the BPT kernels (the same stratified points, seed_seq{seed, pass,
 // pixel, sample + 1}); the reference's painter draws them the same way
 // whichever integrator it runs (painting.cpp:225-257).  Each lane keeps its
@@ -237,8 +248,10 @@ __device__ float pt_brdf_channel(const BrdfTerms& t, const int zero, const Mater
 // memory for a spectrum) and, for RGB, its colour; a spectrum accumulates in
 // the output row.  `estimates` holds 2 * light_count records per thread of
 // the grid.
+inline constexpr int PT_THREADS = 256;
+
 template <int N, typename T, int C>
-__global__ void __launch_bounds__(128, NBPT_PT_MIN_BLOCKS) pt_paths_kernel(
+__global__ void __launch_bounds__(PT_THREADS) pt_paths_kernel(
         const DeviceScene<N, T, 1> scene,
         const Material<T, C>* __restrict__ materials,
         const Light<N, T, C>* __restrict__ lights,
@@ -265,26 +278,33 @@ __global__ void __launch_bounds__(128, NBPT_PT_MIN_BLOCKS) pt_paths_kernel(
         QueryCounters counters{0, 0, 0, 0};
         const SceneQueries<N, T, 1> q{scene, counters};
         Pcg g{0, 0};
+        extern __shared__ __align__(16) unsigned char stacks[];
+        using W = WarpQueries<N, T, 1>;
+        const W warp{q, GroupQueries<N, T, 1>{q, WideStack<T>::of_group(stacks, scene.wide_stack, PT_THREADS)}};
         const Pt<N, T> pt{q, scene, g, Bpt<N, T, 1>{q, scene, g, 0, nullptr, nullptr}};
         Ray<N, T> ray;
         Vec<N, T> gn;
         Color<IN_REGISTERS ? C : 1> reg;
         Color<C> beta;
-        int depth = -1;   // the bounce whose hit is traced next; -1: the primary ray
+        constexpr int STARTS = -2;
+        int depth = STARTS; // the bounce whose hit is traced next; -1: the primary ray, STARTS: a path to be started
         long long i = -1; // the lane's path; -1 when it takes the next one
+        bool done = false;
         while (true)
         {
-                if (i < 0)
+                if (i < 0 && !done)
                 {
-                        if (cancelled(cancel))
-                        {
-                                break;
-                        }
-                        i = reserve_together(next_path, 1);
-                        if (i >= paths)
-                        {
-                                break;
-                        }
+                        i = cancelled(cancel) ? paths : reserve_together(next_path, 1);
+                        done = i >= paths;
+                        i = done ? -1 : i;
+                }
+                if (__syncthreads_and(done ? 1 : 0) != 0)
+                {
+                        break;
+                }
+                const bool live = i >= 0;
+                if (live && depth == STARTS)
+                {
                         // 32-bit index arithmetic: a chunk's path index and a
                         // screen's pixel index fit in 31 bits (the painter's chunk
                         // limits and its screen check), and a 64-bit division costs
@@ -314,21 +334,21 @@ __global__ void __launch_bounds__(128, NBPT_PT_MIN_BLOCKS) pt_paths_kernel(
 
                 float* const out = colors + i * C;
                 Normals<N, T> normals;
-                const Hit<N, T> surface = q.scene_intersect(depth < 0 ? nullptr : &gn, ray, normals);
-                if (depth < 0)
+                const Hit<N, T> surface = warp.scene_intersect(live, depth >= 0, gn, ray, normals);
+                __syncthreads();
+                const bool background = live && depth < 0 && !surface;
+                if (background)
                 {
-                        if (!surface)
-                        {
 #pragma unroll 8
-                                for (int c = 0; c < C; ++c)
-                                {
-                                        out[c] = 0.0f;
-                                }
-                                lum[i] = 0.0f;
-                                valid[i] = 0;
-                                i = -1;
-                                continue;
+                        for (int c = 0; c < C; ++c)
+                        {
+                                out[c] = 0.0f;
                         }
+                        lum[i] = 0.0f;
+                        valid[i] = 0;
+                }
+                else if (live && depth < 0)
+                {
                         // the emitted radiance seen by the primary ray
                         // (LightSource::leave_radiance(-dir))
                         const int li = q.light(surface);
@@ -352,43 +372,70 @@ __global__ void __launch_bounds__(128, NBPT_PT_MIN_BLOCKS) pt_paths_kernel(
 
                 // one bounce (pt.cpp:68-111); the path ends where the
                 // reference's loop breaks
-                bool go_on = static_cast<bool>(surface);
+                bool go_on = live && !background && static_cast<bool>(surface);
                 const Vec<N, T> v = -ray.dir;
                 if (go_on)
                 {
                         go_on = !(dot(normals.shading, v) <= 0);
                 }
+                // direct_lighting (direct_lighting.cpp:150-167): both
+                // estimates of every light, summed in that order
+                int count = 0;
+                for (int k = 0; k < scene.light_count; ++k)
+                {
+                        count += pt.light_with_mis(warp, go_on, k, surface, v, normals, est[count]) ? 1 : 0;
+                        __syncthreads();
+                        count += pt.surface_with_mis(warp, go_on, k, surface, v, normals, est[count]) ? 1 : 0;
+                        __syncthreads();
+                }
                 if (go_on)
                 {
-                        // direct_lighting (direct_lighting.cpp:150-167): both
-                        // estimates of every light, summed in that order
-                        int count = 0;
-                        for (int k = 0; k < scene.light_count; ++k)
-                        {
-                                count += pt.light_with_mis(k, surface, v, normals, est[count]) ? 1 : 0;
-                                count += pt.surface_with_mis(k, surface, v, normals, est[count]) ? 1 : 0;
-                        }
                         const Material<T, C>& m = materials[q.material(surface)];
                         if (count > 0)
                         {
-#pragma unroll 4
-                                for (int c = 0; c < C; ++c)
+                                // four channels at a time: a spectrum's row is
+                                // read and written 16 bytes at a time
+                                constexpr int G = IN_REGISTERS ? 1 : 4;
+#pragma unroll 1
+                                for (int first = 0; first < C; first += IN_REGISTERS ? C : G)
                                 {
-                                        float d = 0.0f;
+                                        constexpr int M = IN_REGISTERS ? C : G;
+                                        float sum[M];
+#pragma unroll
+                                        for (int j = 0; j < M; ++j)
+                                        {
+                                                sum[j] = 0.0f;
+                                        }
                                         for (int e = 0; e < count; ++e)
                                         {
-                                                const PtEstimate& r = est[e];
-                                                const float brdf = pt_brdf_channel(r.terms, r.zero, m, c, sc);
-                                                const float x = (brdf * lights[r.light].radiance.c[c]) * r.scale;
-                                                d = e == 0 ? x : d + x;
+                                                const PtEstimate r = est[e];
+                                                const Light<N, T, C>& l = lights[r.light];
+#pragma unroll
+                                                for (int j = 0; j < M; ++j)
+                                                {
+                                                        const int c = first + j;
+                                                        const float brdf = pt_brdf_channel(r.terms, r.zero, m, c, sc);
+                                                        const float x = (brdf * l.radiance.c[c]) * r.scale;
+                                                        sum[j] = e == 0 ? x : sum[j] + x;
+                                                }
                                         }
                                         if constexpr (IN_REGISTERS)
                                         {
-                                                reg.c[c] += beta.c[c] * d;
+#pragma unroll
+                                                for (int j = 0; j < M; ++j)
+                                                {
+                                                        reg.c[j] += beta.c[j] * sum[j];
+                                                }
                                         }
                                         else
                                         {
-                                                out[c] += beta.c[c] * d;
+                                                float4* const row = reinterpret_cast<float4*>(out + first);
+                                                float4 o = *row;
+                                                o.x += beta.c[first] * sum[0];
+                                                o.y += beta.c[first + 1] * sum[1];
+                                                o.z += beta.c[first + 2] * sum[2];
+                                                o.w += beta.c[first + 3] * sum[3];
+                                                *row = o;
                                         }
                                 }
                         }
@@ -436,6 +483,17 @@ __global__ void __launch_bounds__(128, NBPT_PT_MIN_BLOCKS) pt_paths_kernel(
                                 }
                         }
                 }
+                if (!live)
+                {
+                        continue;
+                }
+                const long long path = i;
+                i = -1;
+                depth = STARTS;
+                if (background)
+                {
+                        continue;
+                }
 
                 // the path is done
                 if constexpr (IN_REGISTERS)
@@ -445,7 +503,7 @@ __global__ void __launch_bounds__(128, NBPT_PT_MIN_BLOCKS) pt_paths_kernel(
                         {
                                 out[c] = reg.c[c];
                         }
-                        lum[i] = luminance(reg, cie_y);
+                        lum[path] = luminance(reg, cie_y);
                         if (!all_finite(reg.c))
                         {
                                 atomicAdd(&stats->nonfinite, 1ull);
@@ -459,14 +517,13 @@ __global__ void __launch_bounds__(128, NBPT_PT_MIN_BLOCKS) pt_paths_kernel(
                         {
                                 final_color.c[c] = out[c];
                         }
-                        lum[i] = luminance(final_color, cie_y);
+                        lum[path] = luminance(final_color, cie_y);
                         if (!all_finite(final_color.c))
                         {
                                 atomicAdd(&stats->nonfinite, 1ull);
                         }
                 }
-                valid[i] = 1;
-                i = -1;
+                valid[path] = 1;
         }
         add_counters(counters, stats);
 }

@@ -262,164 +262,11 @@ struct SceneQueries final
         const DeviceScene<N, T, C>& s;
         QueryCounters& counters;
 
-        // Closest facet of one mesh hit by the ray with t < max_distance
-        // (bvh.h:108-149 traversal, spatial/ray_intersection.h:30-54 leaves).
-        NBPT_CALL int mesh_closest(const MeshShape<N, T>& mesh, const Ray<N, T>& ray, T& distance) const
-        {
-                Vec<N, T> rec;
-                unsigned neg = 0;
-#pragma unroll
-                for (int i = 0; i < N; ++i)
-                {
-                        rec[i] = (ray.dir[i] == 0) ? infinity<T>() : (1 / ray.dir[i]);
-                        if (ray.dir[i] < 0)
-                        {
-                                neg |= 1u << i;
-                        }
-                }
-                const BvhNode<N, T>* const nodes = s.nodes + mesh.node_offset;
-                const std::uint32_t* const indices = s.indices + mesh.index_offset;
-                const Facet<N, T>* const facets = s.facets + mesh.facet_offset;
-
-                std::uint32_t stack[host::BVH_MAX_DEPTH];
-                int top = 0;
-                std::uint32_t node_index = 0;
-                int result = -1;
-                while (true)
-                {
-                        const BvhNode<N, T>& node = nodes[node_index];
-                        ++counters.nodes;
-                        bool descend = false;
-                        if (box_hit<N>(node.lo, node.hi, ray.org, rec, neg, distance))
-                        {
-                                if (node.count == 0)
-                                {
-                                        if (top == host::BVH_MAX_DEPTH)
-                                        {
-                                                // the builders refuse trees this deep; end the
-                                                // query rather than write past the stack
-                                                ++counters.overflows;
-                                                break;
-                                        }
-                                        if ((neg >> node.axis) & 1u)
-                                        {
-                                                stack[top++] = node_index + 1;
-                                                node_index = node.offset;
-                                        }
-                                        else
-                                        {
-                                                stack[top++] = node.offset;
-                                                ++node_index;
-                                        }
-                                        descend = true;
-                                }
-                                else
-                                {
-                                        T min_distance = distance;
-                                        int closest = -1;
-                                        for (int k = 0; k < node.count; ++k)
-                                        {
-                                                const std::uint32_t f = indices[node.offset + k];
-                                                ++counters.facets;
-                                                const T t = facets[f].simplex.intersect(ray);
-                                                if (t > 0 && t < min_distance)
-                                                {
-                                                        min_distance = t;
-                                                        closest = f;
-                                                }
-                                        }
-                                        if (closest >= 0)
-                                        {
-                                                distance = min_distance;
-                                                result = closest;
-                                        }
-                                }
-                        }
-                        if (!descend)
-                        {
-                                if (top == 0)
-                                {
-                                        break;
-                                }
-                                node_index = stack[--top];
-                        }
-                }
-                return result < 0 ? -1 : result + mesh.facet_offset;
-        }
-
-        NBPT_CALL bool mesh_any(const MeshShape<N, T>& mesh, const Ray<N, T>& ray, const T max_distance) const
-        {
-                Vec<N, T> rec;
-                unsigned neg = 0;
-#pragma unroll
-                for (int i = 0; i < N; ++i)
-                {
-                        rec[i] = (ray.dir[i] == 0) ? infinity<T>() : (1 / ray.dir[i]);
-                        if (ray.dir[i] < 0)
-                        {
-                                neg |= 1u << i;
-                        }
-                }
-                const BvhNode<N, T>* const nodes = s.nodes + mesh.node_offset;
-                const std::uint32_t* const indices = s.indices + mesh.index_offset;
-                const Facet<N, T>* const facets = s.facets + mesh.facet_offset;
-
-                std::uint32_t stack[host::BVH_MAX_DEPTH];
-                int top = 0;
-                std::uint32_t node_index = 0;
-                while (true)
-                {
-                        const BvhNode<N, T>& node = nodes[node_index];
-                        ++counters.nodes;
-                        bool descend = false;
-                        if (box_hit<N>(node.lo, node.hi, ray.org, rec, neg, max_distance))
-                        {
-                                if (node.count == 0)
-                                {
-                                        if (top == host::BVH_MAX_DEPTH)
-                                        {
-                                                // the builders refuse trees this deep; end the
-                                                // query rather than write past the stack
-                                                ++counters.overflows;
-                                                return false;
-                                        }
-                                        if ((neg >> node.axis) & 1u)
-                                        {
-                                                stack[top++] = node_index + 1;
-                                                node_index = node.offset;
-                                        }
-                                        else
-                                        {
-                                                stack[top++] = node.offset;
-                                                ++node_index;
-                                        }
-                                        descend = true;
-                                }
-                                else
-                                {
-                                        for (int k = 0; k < node.count; ++k)
-                                        {
-                                                ++counters.facets;
-                                                const T t = facets[indices[node.offset + k]].simplex.intersect(ray);
-                                                if (t > 0 && t < max_distance)
-                                                {
-                                                        return true;
-                                                }
-                                        }
-                                }
-                        }
-                        if (!descend)
-                        {
-                                if (top == 0)
-                                {
-                                        return false;
-                                }
-                                node_index = stack[--top];
-                        }
-                }
-        }
-
-        // The flat and solid shapes of intersect(): closest hit before `best`.
+        // A closest-hit query (scene.cpp:70-95, 97-123, 161-178) moves the
+        // origin off the surface the ray leaves (offset_ray_org), counts itself,
+        // and asks the flat and solid shapes, then the meshes (wide_bvh.cuh).
+        //
+        // The flat and solid shapes: closest hit before `best`.
         __device__ void closest_shape(const Ray<N, T>& ray, T& best, int& kind, int& index) const
         {
                 for (int i = 0; i < s.flat_count; ++i)
@@ -461,7 +308,7 @@ struct SceneQueries final
                 return false;
         }
 
-        // The hit point of intersect(), from the (offset) ray.
+        // The hit point of a query, from the (offset) ray.
         __device__ Vec<N, T> hit_point(const Hit<N, T>& hit, const Ray<N, T>& ray) const
         {
                 const Vec<N, T> p = ray.point(hit.distance);
@@ -476,81 +323,8 @@ struct SceneQueries final
                 }
         }
 
-        // Closest hit of the ray against every shape with t < max_distance,
-        // after moving the origin off the surface it leaves
-        // (scene.cpp:70-95, 97-123, 161-178).
-        NBPT_CALL Hit<N, T> intersect(const Vec<N, T>* geometric_normal, Ray<N, T> ray, T max_distance) const
-        {
-                ++counters.queries;
-                if (geometric_normal)
-                {
-                        ray.org = offset_ray_org(*geometric_normal, ray);
-                }
-                Hit<N, T> hit;
-                hit.kind = static_cast<int>(HitKind::NONE);
-                hit.index = -1;
-                T best = max_distance;
-                for (int i = 0; i < s.flat_count; ++i)
-                {
-                        ++counters.shapes;
-                        const T t = s.flat[i].shape.intersect(ray);
-                        if (t > 0 && t < best)
-                        {
-                                best = t;
-                                hit.kind = static_cast<int>(HitKind::FLAT);
-                                hit.index = i;
-                        }
-                }
-                for (int i = 0; i < s.solid_count; ++i)
-                {
-                        ++counters.shapes;
-                        const T t = s.solid[i].shape.intersect_volume(ray, best);
-                        if (t >= 0 && t < best)
-                        {
-                                best = t;
-                                hit.kind = static_cast<int>(HitKind::SOLID);
-                                hit.index = i;
-                        }
-                }
-                for (int i = 0; i < s.mesh_count; ++i)
-                {
-                        const MeshShape<N, T>& mesh = s.meshes[i];
-                        // the mesh's bound is its root box entry (shapes/mesh.cpp:225-229)
-                        if (box_volume<N>(mesh.lo, mesh.hi, ray, best) < 0)
-                        {
-                                continue;
-                        }
-                        T distance = best;
-                        const int f = mesh_closest(mesh, ray, distance);
-                        if (f >= 0)
-                        {
-                                best = distance;
-                                hit.kind = static_cast<int>(HitKind::FACET);
-                                hit.index = f;
-                        }
-                }
-                if (!hit)
-                {
-                        return hit;
-                }
-                hit.distance = best;
-                const Vec<N, T> p = ray.point(best);
-                switch (static_cast<HitKind>(hit.kind))
-                {
-                case HitKind::FLAT:
-                        hit.point = s.flat[hit.index].shape.plane.project(p);
-                        break;
-                case HitKind::SOLID:
-                        hit.point = s.solid[hit.index].shape.project(p);
-                        break;
-                default:
-                        hit.point = s.facets[hit.index].simplex.plane.project(p);
-                        break;
-                }
-                return hit;
-        }
-
-        // The flat and solid shapes of intersect_any().
+        // The flat and solid shapes of an any-hit query (scene.cpp:125-133,
+        // 180-189).
         __device__ bool any_shape(const Ray<N, T>& ray, const T max_distance) const
         {
                 for (int i = 0; i < s.flat_count; ++i)
@@ -567,47 +341,6 @@ struct SceneQueries final
                         ++counters.shapes;
                         const T t = s.solid[i].shape.intersect_volume(ray, max_distance);
                         if (t >= 0 && t < max_distance)
-                        {
-                                return true;
-                        }
-                }
-                return false;
-        }
-
-        // Any hit with t < max_distance (scene.cpp:125-133, 180-189).
-        NBPT_CALL bool intersect_any(const Vec<N, T>* geometric_normal, Ray<N, T> ray, const T max_distance) const
-        {
-                ++counters.queries;
-                if (geometric_normal)
-                {
-                        ray.org = offset_ray_org(*geometric_normal, ray);
-                }
-                for (int i = 0; i < s.flat_count; ++i)
-                {
-                        ++counters.shapes;
-                        const T t = s.flat[i].shape.intersect(ray);
-                        if (t > 0 && t < max_distance)
-                        {
-                                return true;
-                        }
-                }
-                for (int i = 0; i < s.solid_count; ++i)
-                {
-                        ++counters.shapes;
-                        const T t = s.solid[i].shape.intersect_volume(ray, max_distance);
-                        if (t >= 0 && t < max_distance)
-                        {
-                                return true;
-                        }
-                }
-                for (int i = 0; i < s.mesh_count; ++i)
-                {
-                        const MeshShape<N, T>& mesh = s.meshes[i];
-                        if (box_volume<N>(mesh.lo, mesh.hi, ray, max_distance) < 0)
-                        {
-                                continue;
-                        }
-                        if (mesh_any(mesh, ray, max_distance))
                         {
                                 return true;
                         }
@@ -708,41 +441,6 @@ struct SceneQueries final
                         r.shading = r.geometric;
                 }
                 return r;
-        }
-
-        // integrators/com/visibility.h:174-204: a hit whose shading normal
-        // faces away from the ray is re-cast up to two more times.
-        NBPT_CALL Hit<N, T> scene_intersect(const Vec<N, T>* geometric_normal, const Ray<N, T>& ray, Normals<N, T>& normals)
-                const
-        {
-                Hit<N, T> h = intersect(geometric_normal, ray, infinity<T>());
-                if (!h)
-                {
-                        return h;
-                }
-                normals = compute_normals(h, ray.dir);
-                if (dot(ray.dir, normals.shading) <= 0)
-                {
-                        return h;
-                }
-                for (int i = 0; i < 2; ++i)
-                {
-                        const Vec<N, T> g = geometric_normal_of(h);
-                        Ray<N, T> r2 = ray;
-                        r2.org = h.point;
-                        h = intersect(&g, r2, infinity<T>());
-                        if (!h)
-                        {
-                                return h;
-                        }
-                }
-                normals = compute_normals(h, ray.dir);
-                return h;
-        }
-
-        __device__ Vec<N, T> geometric_normal_of(const Hit<N, T>& h) const
-        {
-                return geometric_normal(h);
         }
 };
 } // namespace nbpt

@@ -259,7 +259,7 @@ __global__ void __launch_bounds__(WALK_THREADS) walk_begin_kernel(
 }
 
 // Eight lanes per queued ray: the closest hit among the meshes, and the
-// re-casts of scene_intersect() (integrators/com/visibility.h:174-204) for a
+// re-casts (integrators/com/visibility.h:174-204) for a
 // facet whose interpolated normal faces away from the ray; only facets have
 // one.  The list then holds the last query's hit and its ray's origin.
 template <int N, typename T>

@@ -235,8 +235,7 @@ struct GroupQueries final
                 return threadIdx.x % 32 / WIDE * WIDE;
         }
 
-        // The flat and solid shapes of SceneQueries::intersect(), a shape to
-        // a lane: the closest hit before `best`, the first of several at one
+        // The flat and solid shapes of a query, a shape to a lane: the closest hit before `best`, the first of several at one
         // distance; (ANY) whether there is one, in `kind`.
         template <bool ANY>
         __device__ void shapes(const bool active, const Ray<N, T>& ray, T& best, int& kind, int& index) const
@@ -292,8 +291,7 @@ struct GroupQueries final
                 }
         }
 
-        // The meshes of SceneQueries::intersect(): the closest hit before
-        // `best`, or (ANY) whether there is one, in `kind`.
+        // The meshes of a query: the closest hit before `best`, or (ANY) whether there is one, in `kind`.
         template <bool ANY>
         __device__ void mesh(const bool active, const Ray<N, T>& ray, T& best, int& kind, int& index) const
         {
@@ -546,6 +544,159 @@ private:
         __device__ static double slab_min(const double far, const double a)
         {
                 return a < far ? a : far;
+        }
+};
+
+// ---------------------------------------------------------------------------
+// queries of a ray per lane, for kernels that keep a path on a lane: the warp
+// calls them together.  The lanes test the flat and solid shapes; then the
+// rays that may enter a mesh (one in five) go to the warp's four groups, four
+// at a time, through shuffles.
+template <int N, typename T, int C>
+struct WarpQueries final
+{
+        static constexpr unsigned FULL = 0xffffffffu;
+
+        const SceneQueries<N, T, C>& q;
+        const GroupQueries<N, T, C> group;
+
+        struct MeshHit final
+        {
+                T distance;
+                int kind;
+                int index;
+        };
+
+        // the meshes of the lanes that want them: the closest hit before
+        // `best` (ANY: whether there is one), kind NONE without
+        template <bool ANY>
+        NBPT_CALL MeshHit mesh(const bool wants, const Ray<N, T>& ray, const T best) const
+        {
+                MeshHit mine{best, static_cast<int>(HitKind::NONE), -1};
+                const int lane = static_cast<int>(threadIdx.x & 31);
+                const int my_group = lane / WIDE;
+                unsigned pending = __ballot_sync(FULL, wants);
+                while (pending != 0)
+                {
+                        // group g takes the g-th pending lane
+                        unsigned rest = pending;
+                        for (int g = 0; g < my_group; ++g)
+                        {
+                                rest &= rest - 1;
+                        }
+                        const bool active = rest != 0;
+                        const int from = active ? __ffs(static_cast<int>(rest)) - 1 : 0;
+                        Ray<N, T> r;
+#pragma unroll
+                        for (int k = 0; k < N; ++k)
+                        {
+                                r.org[k] = __shfl_sync(FULL, ray.org[k], from);
+                                r.dir[k] = __shfl_sync(FULL, ray.dir[k], from);
+                        }
+                        T distance = __shfl_sync(FULL, best, from);
+                        int kind = static_cast<int>(HitKind::NONE);
+                        int index = -1;
+                        group.template mesh<ANY>(active, r, distance, kind, index);
+                        // back to the ray's lane
+                        const int place = __popc(pending & ((1u << lane) - 1));
+                        const int to = (place % (32 / WIDE)) * WIDE;
+                        const T d = __shfl_sync(FULL, distance, to);
+                        const int k = __shfl_sync(FULL, kind, to);
+                        const int x = __shfl_sync(FULL, index, to);
+                        if (((pending >> lane) & 1u) != 0 && place < 32 / WIDE)
+                        {
+                                mine = {d, k, x};
+                        }
+#pragma unroll
+                        for (int g = 0; g < 32 / WIDE; ++g)
+                        {
+                                pending &= pending - 1;
+                        }
+                }
+                return mine;
+        }
+
+        // a closest-hit query from an offset origin
+        __device__ Hit<N, T> closest(const bool active, const Ray<N, T>& ray, const T max_distance) const
+        {
+                Hit<N, T> h;
+                h.kind = static_cast<int>(HitKind::NONE);
+                h.index = -1;
+                h.distance = max_distance;
+                bool wants = false;
+                if (active)
+                {
+                        ++q.counters.queries;
+                        q.closest_shape(ray, h.distance, h.kind, h.index);
+                        wants = q.enters_mesh(ray, h.distance);
+                }
+                const MeshHit m = mesh<false>(wants, ray, h.distance);
+                if (m.kind != static_cast<int>(HitKind::NONE))
+                {
+                        h.distance = m.distance;
+                        h.kind = m.kind;
+                        h.index = m.index;
+                }
+                if (h)
+                {
+                        h.point = q.hit_point(h, ray);
+                }
+                return h;
+        }
+
+        // an any-hit query from an offset origin
+        __device__ bool any(const bool active, const Ray<N, T>& ray, const T max_distance) const
+        {
+                bool hit = false;
+                bool wants = false;
+                if (active)
+                {
+                        ++q.counters.queries;
+                        hit = q.any_shape(ray, max_distance);
+                        wants = !hit && q.enters_mesh(ray, max_distance);
+                }
+                const MeshHit m = mesh<true>(wants, ray, max_distance);
+                return hit || m.kind != static_cast<int>(HitKind::NONE);
+        }
+
+        // scene_intersect (integrators/com/visibility.h:174-204): a hit whose
+        // shading normal faces away from the ray is re-cast up to two more times;
+        // `normal`: of the surface the ray leaves, where there is one
+        __device__ Hit<N, T> scene_intersect(const bool active, const bool from_surface, const Vec<N, T>& normal,
+                                             const Ray<N, T>& from, Normals<N, T>& normals) const
+        {
+                Ray<N, T> ray = from;
+                if (active && from_surface)
+                {
+                        ray.org = offset_ray_org(normal, from);
+                }
+                Hit<N, T> h = closest(active, ray, infinity<T>());
+                bool recast = false;
+                if (active && h)
+                {
+                        normals = q.compute_normals(h, from.dir);
+                        recast = dot(from.dir, normals.shading) > 0;
+                }
+                const bool moved = recast;
+                for (int i = 0; i < 2 && __any_sync(FULL, recast); ++i)
+                {
+                        if (recast)
+                        {
+                                ray.org = h.point;
+                                ray.org = offset_ray_org(q.geometric_normal(h), ray);
+                        }
+                        const Hit<N, T> next = closest(recast, ray, infinity<T>());
+                        if (recast)
+                        {
+                                h = next;
+                        }
+                        recast = recast && static_cast<bool>(h);
+                }
+                if (moved && h)
+                {
+                        normals = q.compute_normals(h, from.dir);
+                }
+                return h;
         }
 };
 } // namespace nbpt
