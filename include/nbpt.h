@@ -241,8 +241,8 @@ typedef struct nbpt_painter_options
         int slab_begin;
         int slab_end;
         int pixel_sums; /* NBPT_PIXEL_SUMS_* */
-        /* device bytes of the per-chunk path buffers (0: a fifth of the
-         * device's memory within [4, 32] GiB); a pass runs its paths in
+        /* device bytes of the per-chunk path buffers (0: a tenth of the
+         * device's memory within [4, 16] GiB); a pass runs its paths in
          * chunks of as many as they hold, with the same images whatever the
          * size */
         long long chunk_budget;

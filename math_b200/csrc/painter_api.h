@@ -130,8 +130,8 @@ public:
                                                         int slab_end = -1, bool flat_shading = false,
                                                         long long chunk_budget = 0, int pixel_sums = 0) = 0;
         // device bytes create_painter would allocate.  chunk_budget: bytes
-        // for the buffers of one chunk of paths (0: a fifth of the device's
-        // memory within [4, 32] GiB); the job server gives each of its slots
+        // for the buffers of one chunk of paths (0: a tenth of the device's
+        // memory within [4, 16] GiB); the job server gives each of its slots
         // a share of its memory budget
         virtual long long painter_bytes(int samples_per_pixel, int max_depth,
                                         Integrator integrator = Integrator::BPT,

@@ -2633,14 +2633,16 @@ class PainterT final : public Painter
         int launches_accumulate_ = 0;
         Statistics statistics_{};
 
-        // Device memory for the per-path buffers of one chunk.  The walk and
-        // connect kernels are persistent over a chunk, and every chunk ends in
-        // a tail in which the last, longest paths run on an emptying GPU;
-        // larger chunks make the tails rarer.  Measured on five jobs of the
-        // mixed batch (3/4/5-space, one pass each): 4 -> 16 GiB 1.09-1.41x
-        // faster per pass, 4 -> 32 GiB 1.11-1.53x.  A fifth of the device's
-        // memory, within [4, 32] GiB (NBPT_CHUNK_BUDGET_GB, when defined, sets
-        // it for sweeps).
+        // Device memory for the per-path buffers of one chunk.  A chunk's waves
+        // end with the longest rays of each on an emptying GPU, and every chunk
+        // has some forty launches; larger chunks have fewer of both per path.
+        // Milliseconds of a pass with 4 / 8 / 16 / 32 GiB: 4-space spectral f32
+        // (7.1 M paths) 50.2 / 45.3 / 42.7 / 41.3, 5-space f32 (1.7 M, depth 8)
+        // 21.3 / 16.8 / 13.0 / 12.9, 4-space sphere f32 8.4 / 7.9 / 7.4 / 7.4,
+        // 3-space f64 6.3 / 6.2 / 6.2 / 6.2.  A tenth of the device's memory,
+        // within [4, 16] GiB: twice that gains at most 3 % and doubles what a
+        // first render has to allocate, which takes up to 0.4 s for 32 GiB
+        // (NBPT_CHUNK_BUDGET_GB, when defined, sets it for sweeps).
         static long long chunk_budget()
         {
 #ifdef NBPT_CHUNK_BUDGET_GB
@@ -2659,7 +2661,7 @@ class PainterT final : public Painter
                         std::size_t free = 0;
                         std::size_t total = 0;
                         NBPT_CUDA(cudaMemGetInfo(&free, &total));
-                        b = std::min(32LL << 30, std::max(4LL << 30, static_cast<long long>(total / 5)));
+                        b = std::min(16LL << 30, std::max(4LL << 30, static_cast<long long>(total / 10)));
                         by_device[device] = b;
                 }
                 return b;
