@@ -187,23 +187,15 @@ __global__ void sj_points_kernel(
         }
 }
 
-// Minimum resident blocks of 128 threads per SM asked of the compiler for
-// the path kernels, which caps their registers (65536 / (128 * blocks)), per
-// dimension and precision, from launch-bound sweeps of the mixed-scene
-// batch's jobs on a B200 (one pass each, best of three):
-//   float: 16 blocks (32 registers) in 3-, 4- and 5-space; 12 and 8 blocks
-//          were 1-8 % slower;
-//   double: 8 blocks (64 registers) in 4- and 5-space, 7-8 % faster than 16;
-//          12 blocks in 3-space, 5 % faster than 16.
-// NBPT_PATHS_MIN_BLOCKS, when defined, sets every kernel's (for sweeps).
+// Blocks of 128 threads per SM of the kernels over the strategies: the
+// registers of paths_light_kernel (65536 / (128 * blocks)) and the grid that
+// paths_connect_kernel strides over its queues.  Where these kernels' shape
+// hardly matters the figures of the earlier persistent kernels stand: 16 in
+// single precision, 8 in double (12 in 3-space).
 template <int N, typename T>
 struct PathsMinBlocks final
 {
-#ifdef NBPT_PATHS_MIN_BLOCKS
-        static constexpr int value = NBPT_PATHS_MIN_BLOCKS;
-#else
         static constexpr int value = std::is_same_v<T, double> ? (N == 3 ? 12 : 8) : 16;
-#endif
 };
 
 // ---------------------------------------------------------------------------
