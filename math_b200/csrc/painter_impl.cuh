@@ -166,15 +166,27 @@ public:
         }
 };
 
-// dynamic shared memory beyond 48 KB has to be asked for
+// Lets a kernel take `bytes` of dynamic shared memory.  More than 48 KB has to
+// be asked for, and what is asked for is one value per kernel and device,
+// whichever painter and thread asks.  Every call therefore sets the same one,
+// all that the device gives a block beside the kernel's static shared memory:
+// set to a caller's own need, it would be too small for a launch of another
+// painter that needs more.  What a block gets is what its launch asks for.
 template <typename Kernel>
 void allow_shared(Kernel* const kernel, const std::size_t bytes)
 {
-        if (bytes > 48 * 1024)
+        if (bytes <= 48 * 1024)
         {
-                NBPT_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               static_cast<int>(bytes)));
+                return;
         }
+        int device = 0;
+        int limit = 0;
+        cudaFuncAttributes attributes{};
+        NBPT_CUDA(cudaGetDevice(&device));
+        NBPT_CUDA(cudaDeviceGetAttribute(&limit, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
+        NBPT_CUDA(cudaFuncGetAttributes(&attributes, kernel));
+        NBPT_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       limit - static_cast<int>(attributes.sharedSizeBytes)));
 }
 
 inline unsigned blocks_for(const long long n, const int threads)
