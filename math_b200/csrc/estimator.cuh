@@ -681,6 +681,189 @@ struct Screen final
         long long source_first = 0;
 };
 
+inline constexpr int neighbours(const int n)
+{
+        return n == 3 ? 9 : (n == 4 ? 27 : 81);
+}
+
+// RGB accumulation of few samples per pixel: a thread per receiving pixel goes
+// through its 3^(n-1) source pixels, forms each group and merges it.  Groups
+// of one to nine samples take less time to form than to carry through memory
+// between the two kernels below (132-152 bytes each), once the screen has
+// enough pixels to fill the GPU with threads.  Milliseconds with this kernel /
+// with the two, single precision: 3-space 8 M pixels x 1 sample 3.4 / 16.4,
+// 160,000 x 9 0.24 / 0.40 and 40,000 x 9 0.125 / 0.125; 4-space 8 M x 1
+// 8.8 / 49.7, 157,000 x 8 1.06 / 1.15 and 39,000 x 8 0.40 / 0.31; 5-space
+// 2.6 M x 1 9.5 / 55.9.  From sixteen samples on the two are faster at every
+// size (3-space 2.5 M x 16 7.1 / 5.9, 5-space 2.6 M x 16 89.9 / 65.1).
+//
+// The screens where both are about equally fast, but for a single sample per
+// pixel (no sums and no order), have some 600 pixels per sample of a pixel's
+// neighbourhood: 3-space x 4 15,000 to 20,000, x 9 40,000 to 55,000, 4-space
+// x 8 110,000 (single) to 300,000 (double).
+template <int N>
+inline constexpr bool thread_per_pixel(const long long pixels, const int spp)
+{
+        return spp == 1 || (spp < 16 && pixels >= 600LL * spp * neighbours(N));
+}
+
+// Merge one pass's samples of the 3^(n-1) neighbours into receiving pixel t
+// (global index).
+template <int N, typename T, int C, typename S>
+NBPT_HD void accumulate_pixel(
+        const Screen<N>& screen,
+        const long long t,
+        const int spp,
+        const T* __restrict__ points,
+        const float* __restrict__ colors,
+        const float* __restrict__ lum,
+        const unsigned char* __restrict__ valid,
+        const T alpha,
+        const T exp_radius,
+        PixelState<C, S>& st)
+{
+        int tc[N - 1];
+        {
+                long long rest = t;
+#pragma unroll
+                for (int d = 0; d < N - 1; ++d)
+                {
+                        tc[d] = static_cast<int>(rest % screen.size[d]);
+                        rest /= screen.size[d];
+                }
+        }
+
+        float w[MAX_GROUP];
+        int color_order[MAX_GROUP];
+        float background[MAX_GROUP];
+
+        // sources in increasing pixel index: the last screen axis outermost
+        for (int nb = 0; nb < neighbours(N); ++nb)
+        {
+                int pc[N - 1];
+                bool inside = true;
+                {
+                        int rest = nb;
+#pragma unroll
+                        for (int d = 0; d < N - 1; ++d)
+                        {
+                                pc[d] = tc[d] + (rest % 3) - 1;
+                                rest /= 3;
+                                inside = inside && pc[d] >= 0 && pc[d] < screen.size[d];
+                        }
+                }
+                if (!inside)
+                {
+                        continue;
+                }
+                long long p = 0;
+#pragma unroll
+                for (int d = N - 2; d >= 0; --d)
+                {
+                        p = p * screen.size[d] + pc[d];
+                }
+
+                // weights (pixel_filter.h:57-69, gaussian.h:66-77) and the
+                // selection of colour and background samples (com/select.h:28-47)
+                int nc = 0;
+                int nbg = 0;
+                for (int j = 0; j < spp; ++j)
+                {
+                        const long long sidx = (p - screen.source_first) * spp + j;
+                        const T x0 = (static_cast<T>(tc[0] - pc[0]) + T(0.5)) - points[sidx * (N - 1)];
+                        T weight = max_value(T(0), exp(alpha * x0 * x0) - exp_radius);
+#pragma unroll
+                        for (int d = 1; d < N - 1; ++d)
+                        {
+                                const T x = (static_cast<T>(tc[d] - pc[d]) + T(0.5)) - points[sidx * (N - 1) + d];
+                                weight *= max_value(T(0), exp(alpha * x * x) - exp_radius);
+                        }
+                        if (!(weight > 0))
+                        {
+                                continue;
+                        }
+                        const float wf = static_cast<float>(weight);
+                        if (valid[sidx])
+                        {
+                                w[j] = wf;
+                                color_order[nc++] = j;
+                        }
+                        else
+                        {
+                                background[nbg++] = wf;
+                        }
+                }
+
+                if (nc > 0)
+                {
+                        const float* const source_lum = lum + (p - screen.source_first) * spp;
+                        order_group(color_order, nc, [&](const int i) { return w[i] * source_lum[i]; });
+                        const ColorGroup<C> g{colors + (p - screen.source_first) * spp * C, w, source_lum, color_order, nc, C, 1, 0};
+                        S g_sum[C];
+                        S g_wsum = 0;
+#pragma unroll 8
+                        for (int c = 0; c < C; ++c)
+                        {
+                                g_sum[c] = 0;
+                        }
+                        const bool g_full = nc > HELD_OUT;
+                        if (g_full)
+                        {
+                                // create_with_sum (samples/com/create.h:28-55)
+                                for (int k = HELD_OUT / 2; k < nc - HELD_OUT / 2; ++k)
+                                {
+#pragma unroll 8
+                                        for (int c = 0; c < C; ++c)
+                                        {
+                                                g_sum[c] += g.color(k, c);
+                                        }
+                                        g_wsum += w[color_order[k]];
+                                }
+                        }
+                        merge_color_group(st.color, g, g_sum, g_wsum, g_full);
+                }
+                if (nbg > 0)
+                {
+                        // background samples are ordered by value
+                        int order[MAX_GROUP];
+                        for (int k = 0; k < nbg; ++k)
+                        {
+                                order[k] = k;
+                        }
+                        order_group(order, nbg, [&](const int i) { return background[i]; });
+                        float sorted[MAX_GROUP];
+                        for (int k = 0; k < nbg; ++k)
+                        {
+                                sorted[k] = background[order[k]];
+                        }
+                        merge_background_group(st.background, sorted, nbg);
+                }
+        }
+}
+
+template <int N, typename T, int C, typename S>
+__global__ void __launch_bounds__(128) accumulate_kernel(
+        const Screen<N> screen,
+        const long long pixel_count,
+        const int spp,
+        const T* __restrict__ points,
+        const float* __restrict__ colors,
+        const float* __restrict__ lum,
+        const unsigned char* __restrict__ valid,
+        const T alpha,
+        const T exp_radius,
+        PixelState<C, S>* __restrict__ state)
+{
+        const long long t = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
+        if (t >= pixel_count)
+        {
+                return;
+        }
+        PixelState<C, S> st = state[t];
+        accumulate_pixel<N, T, C, S>(screen, screen.first + t, spp, points, colors, lum, valid, alpha, exp_radius, st);
+        state[t] = st;
+}
+
 // RGB accumulation in two kernels: the group of every (source pixel,
 // receiving pixel) pair is formed by a thread of its own (group_kernel), then
 // every receiving pixel merges its groups in increasing source index
@@ -696,11 +879,6 @@ struct Screen final
 // lanes read the same samples of the same source.  A group travels as a
 // sample set (120-152 bytes).  Those 4,096 pixels now take 0.15 ms to form
 // and 0.27 ms to merge, 105,000 of 16 samples 1.2 and 1.4 ms (4.5 before).
-
-inline constexpr int neighbours(const int n)
-{
-        return n == 3 ? 9 : (n == 4 ? 27 : 81);
-}
 
 // threads of a group_kernel block and the source pixels they share
 template <int N>

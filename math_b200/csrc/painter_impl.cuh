@@ -2740,9 +2740,9 @@ public:
                 return std::min(pixels, GROUP_BYTES / static_cast<long long>(neighbours(N) * sizeof(PixelState<3, S>)));
         }
 
-        static long long group_bytes(const long long pixels, const bool sums_in_double)
+        static long long group_bytes(const long long pixels, const int spp, const bool sums_in_double)
         {
-                if constexpr (C != 3)
+                if (C != 3 || thread_per_pixel<N>(pixels, spp))
                 {
                         return 0;
                 }
@@ -2764,7 +2764,7 @@ public:
                                                 : chunk_pixels(pixels, spp, max_depth, integrator, budget) * spp *
                                                           chunk_path_bytes(max_depth);
                 return (strata + 1) * sizeof(T) + samples * per_sample + pixels * per_pixel + sizeof(PathStats) +
-                       chunk + group_bytes(pixels, sums_in_double);
+                       chunk + group_bytes(pixels, spp, sums_in_double);
         }
 
         // slab_end < 0: the whole screen; else the rows [slab_begin, slab_end)
@@ -2855,7 +2855,7 @@ public:
                 {
                         state_.allocate(pixels_);
                 }
-                groups_.allocate(group_bytes(pixels_, double_sums_));
+                groups_.allocate(group_bytes(pixels_, spp_, double_sums_));
                 stats_.allocate(1);
                 NBPT_CUDA(cudaMemsetAsync(stats_.get(), 0, sizeof(PathStats), stream_));
                 cancel_.allocate(1);
@@ -3295,9 +3295,10 @@ public:
                 }
         }
 
-        // RGB: the groups of a range of receiving pixels at a time, as many
-        // as the scratch holds (GROUP_BYTES); the sources of a range reach one
-        // pixel past it along every axis.
+        // RGB: small screens in one launch, few samples per pixel by a thread
+        // per pixel, else the groups of a range of receiving pixels at a time, as
+        // many as the scratch holds (GROUP_BYTES); the sources of a range reach
+        // one pixel past it along every axis.
         template <typename S>
         void accumulate_groups(const Screen<N>& screen, const T alpha, const T exp_radius,
                                PixelState<3, S>* const state)
@@ -3315,9 +3316,18 @@ public:
                         launches_accumulate_ = 1;
                         return;
                 }
+                if (thread_per_pixel<N>(pixels_, spp_))
+                {
+                        accumulate_kernel<N, T, 3, S><<<blocks_for(pixels_, 128), 128, 0, stream_>>>(
+                                screen, pixels_, spp_, points_.get(), colors_.get(), lum_.get(), valid_.get(), alpha,
+                                exp_radius, state);
+                        NBPT_CUDA(cudaGetLastError());
+                        launches_accumulate_ = 1;
+                        return;
+                }
                 const long long range = group_pixels<S>(pixels_);
-                // given back by release_scratch()
-                groups_.allocate_if_smaller(group_bytes(pixels_, double_sums_));
+                // release_scratch() gives it back (of a render that a job server made)
+                groups_.allocate_if_smaller(group_bytes(pixels_, spp_, double_sums_));
                 auto* const groups = reinterpret_cast<PixelState<3, S>*>(groups_.get());
                 long long reach = 0;
                 long long row = 1;
