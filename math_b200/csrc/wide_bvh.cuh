@@ -307,53 +307,74 @@ struct GroupQueries final
                                 neg |= 1u << i;
                         }
                 }
-                for (int m = 0; m < s.mesh_count; ++m)
+                for (int first = 0; first < s.mesh_count; first += WIDE)
                 {
-                        // the mesh's bound is its root box entry (shapes/mesh.cpp:225-229)
-                        const bool enters = active && !(ANY && kind != static_cast<int>(HitKind::NONE)) &&
-                                            !(box_volume<N>(s.meshes[m].lo, s.meshes[m].hi, ray, best) < 0);
-                        if (!__any_sync(FULL, enters))
+                        // a mesh's bound is its root box entry (shapes/mesh.cpp:225-229),
+                        // tested by a lane per mesh: its near side does not depend on
+                        // `best`, with which it is compared when the mesh's turn comes
+                        const int mine = first + static_cast<int>(lane());
+                        T bound = -1;
+                        if (active && !(ANY && kind != static_cast<int>(HitKind::NONE)) && mine < s.mesh_count)
                         {
-                                continue;
+                                bound = box_volume<N>(s.meshes[mine].lo, s.meshes[mine].hi, ray, best);
                         }
-                        int top = 0;
-                        if (enters)
+                        unsigned meshes = (__ballot_sync(FULL, !(bound < 0)) >> group_shift()) & 0xffu;
+                        while (__any_sync(FULL, meshes != 0))
                         {
-                                top = 1;
-                                if (lane() == 0)
+                                const int next = meshes != 0 ? __ffs(static_cast<int>(meshes)) - 1 : 0;
+                                const T near = __shfl_sync(FULL, bound, next, WIDE);
+                                int top = 0;
+                                if (meshes != 0 && near <= best)
                                 {
-                                        stack.near[0] = 0;
-                                        stack.ref[0] = static_cast<std::uint32_t>(m);
-                                }
-                        }
-                        __syncwarp();
-                        while (__any_sync(FULL, top > 0))
-                        {
-                                bool node = false;
-                                std::uint32_t ref = 0;
-                                while (top > 0 && !node)
-                                {
-                                        --top;
-                                        if (!(stack.near[top] <= best))
+                                        top = 1;
+                                        if (lane() == 0)
                                         {
-                                                continue;
-                                        }
-                                        ref = stack.ref[top];
-                                        node = (ref & WIDE_LEAF) == 0;
-                                        if (!ANY && !node && stack.distance[top] < best)
-                                        {
-                                                best = stack.distance[top];
-                                                kind = static_cast<int>(HitKind::FACET);
-                                                index = static_cast<int>(ref & ~WIDE_LEAF);
+                                                stack.near[0] = 0;
+                                                stack.ref[0] = static_cast<std::uint32_t>(first + next);
                                         }
                                 }
-                                __syncwarp(); // the entries are read before they are written again
-                                children<ANY>(node, ref, ray, rec, neg, best, kind, top);
+                                meshes &= meshes - 1;
+                                __syncwarp();
+                                traverse<ANY>(ray, rec, neg, best, kind, index, top);
+                                if (ANY && kind != static_cast<int>(HitKind::NONE))
+                                {
+                                        meshes = 0;
+                                }
                         }
                 }
         }
 
 private:
+        // Visits what is stacked and all that follows from it.
+        template <bool ANY>
+        __device__ void traverse(const Ray<N, T>& ray, const Vec<N, T>& rec, const unsigned neg, T& best, int& kind,
+                                 int& index, int top) const
+        {
+                while (__any_sync(FULL, top > 0))
+                {
+                        bool node = false;
+                        std::uint32_t ref = 0;
+                        while (top > 0 && !node)
+                        {
+                                --top;
+                                if (!(stack.near[top] <= best))
+                                {
+                                        continue;
+                                }
+                                ref = stack.ref[top];
+                                node = (ref & WIDE_LEAF) == 0;
+                                if (!ANY && !node && stack.distance[top] < best)
+                                {
+                                        best = stack.distance[top];
+                                        kind = static_cast<int>(HitKind::FACET);
+                                        index = static_cast<int>(ref & ~WIDE_LEAF);
+                                }
+                        }
+                        __syncwarp(); // the entries are read before they are written again
+                        children<ANY>(node, ref, ray, rec, neg, best, kind, top);
+                }
+        }
+
         // Tests the children of node `ref`, and the facets of those that are
         // leaves, and stacks what is hit, the first to visit on top.  ANY: a
         // facet hit ends the query.
