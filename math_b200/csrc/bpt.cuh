@@ -294,7 +294,8 @@ struct Bpt final
 
         // occluded(scene, normals, ray, distance) (visibility.h:99-123) of a ray
         // per lane; the warp calls it together
-        __device__ bool occluded_ray(const WarpQueries<N, T, C>& warp, const bool active, const Normals<N, T>& normals,
+        template <typename Warp>
+        __device__ bool occluded_ray(const Warp& warp, const bool active, const Normals<N, T>& normals,
                                      const Ray<N, T>& from, const T distance) const
         {
                 bool open = active;
@@ -309,7 +310,7 @@ struct Bpt final
                 }
                 const bool occluded = active && !open;
                 bool ask = open;
-                if (__any_sync(WarpQueries<N, T, C>::FULL, moves))
+                if (__any_sync(Warp::FULL, moves))
                 {
                         // the surface's other side first (move_and_intersect_any,
                         // visibility.h)

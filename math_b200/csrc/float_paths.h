@@ -23,8 +23,9 @@ struct FloatPathKernels final
         decltype(&connect_sight_kernel<N, float>) sight;
         decltype(&paths_replay_kernel<N, float, 3, 1>) replay_rgb;
         decltype(&paths_replay_kernel<N, float, 64, 32>) replay_spectrum;
-        decltype(&pt_paths_kernel<N, float, 3>) pt_rgb;
-        decltype(&pt_paths_kernel<N, float, 64>) pt_spectrum;
+        // [many_shapes()]
+        decltype(&pt_paths_kernel<N, float, 3, false>) pt_rgb[2];
+        decltype(&pt_paths_kernel<N, float, 64, false>) pt_spectrum[2];
 };
 
 template <int N>

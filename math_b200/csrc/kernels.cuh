@@ -537,7 +537,7 @@ __device__ inline void group_closest(const GroupQueries<N, T, 1>& group, const b
                 group.q.counters.queries += G::lane() == 0 ? 1 : 0;
         }
         group.template shapes<false>(active, ray, found.distance, found.kind, found.index);
-        group.template mesh<false>(active, ray, found.distance, found.kind, found.index);
+        group.template mesh<false, false>(active, ray, found.distance, found.kind, found.index);
         if (active)
         {
                 hit = found;
@@ -664,7 +664,7 @@ __global__ void __launch_bounds__(CONNECT_THREADS) connect_sight_kernel(
                         counters.queries += whole && !open && G::lane() == 0 ? 1 : 0;
                         group.template shapes<true>(whole && !open, ray, distance, kind, index);
                 }
-                group.template mesh<true>(!open, ray, distance, kind, index);
+                group.template mesh<true, false>(!open, ray, distance, kind, index);
                 if (kind != static_cast<int>(HitKind::NONE) && G::lane() == 0)
                 {
                         *slot = 0;

@@ -2405,7 +2405,7 @@ __global__ void __launch_bounds__(TRACE_THREADS) trace_kernel(
         if (any)
         {
                 group.template shapes<true>(active, ray, h.distance, h.kind, h.index);
-                group.template mesh<true>(active, ray, h.distance, h.kind, h.index);
+                group.template mesh<true, false>(active, ray, h.distance, h.kind, h.index);
                 if (active && G::lane() == 0)
                 {
                         kind[i] = h ? 1 : 0;
@@ -2413,7 +2413,7 @@ __global__ void __launch_bounds__(TRACE_THREADS) trace_kernel(
                 return;
         }
         group.template shapes<false>(active, ray, h.distance, h.kind, h.index);
-        group.template mesh<false>(active, ray, h.distance, h.kind, h.index);
+        group.template mesh<false, false>(active, ray, h.distance, h.kind, h.index);
         if (!active || G::lane() != 0)
         {
                 return;
@@ -3012,23 +3012,24 @@ public:
                         return &paths_replay_kernel<N, T, C, LANES>;
                 }
         }
-        static auto pt_kernel()
+        auto pt_kernel() const
         {
+                const bool many = many_shapes(scene_->device());
                 if constexpr (std::is_same_v<T, float>)
                 {
                         static_assert(C == 3 || C == 64);
                         if constexpr (C == 3)
                         {
-                                return float_path_kernels<N>().pt_rgb;
+                                return float_path_kernels<N>().pt_rgb[many];
                         }
                         else
                         {
-                                return float_path_kernels<N>().pt_spectrum;
+                                return float_path_kernels<N>().pt_spectrum[many];
                         }
                 }
                 else
                 {
-                        return &pt_paths_kernel<N, T, C>;
+                        return many ? &pt_paths_kernel<N, T, C, true> : &pt_paths_kernel<N, T, C, false>;
                 }
         }
 

@@ -115,7 +115,8 @@ struct Pt final
 
         // sample_light_with_mis (direct_lighting.cpp:59-99); the lights here
         // are area lights (is_delta() false).  The warp calls it together.
-        __device__ bool light_with_mis(const WarpQueries<N, T, 1>& warp, const bool active, const int k,
+        template <typename Warp>
+        __device__ bool light_with_mis(const Warp& warp, const bool active, const int k,
                                        const Hit<N, T>& surface, const Vec<N, T>& v, const Normals<N, T>& normals,
                                        PtEstimate& out) const
         {
@@ -157,7 +158,8 @@ struct Pt final
 
         // sample_surface_with_mis (direct_lighting.cpp:101-147); no shape
         // here is specular.  The warp calls it together.
-        __device__ bool surface_with_mis(const WarpQueries<N, T, 1>& warp, const bool active, const int k,
+        template <typename Warp>
+        __device__ bool surface_with_mis(const Warp& warp, const bool active, const int k,
                                          const Hit<N, T>& surface, const Vec<N, T>& v, const Normals<N, T>& normals,
                                          PtEstimate& out) const
         {
@@ -250,7 +252,7 @@ __device__ float pt_brdf_channel(const BrdfTerms& t, const int zero, const Mater
 // the grid.
 inline constexpr int PT_THREADS = 256;
 
-template <int N, typename T, int C>
+template <int N, typename T, int C, bool MANY>
 __global__ void __launch_bounds__(PT_THREADS) pt_paths_kernel(
         const DeviceScene<N, T, 1> scene,
         const Material<T, C>* __restrict__ materials,
@@ -279,7 +281,7 @@ __global__ void __launch_bounds__(PT_THREADS) pt_paths_kernel(
         const SceneQueries<N, T, 1> q{scene, counters};
         Pcg g{0, 0};
         extern __shared__ __align__(16) unsigned char stacks[];
-        using W = WarpQueries<N, T, 1>;
+        using W = WarpQueries<N, T, 1, MANY>;
         const W warp{q, GroupQueries<N, T, 1>{q, WideStack<T>::of_group(stacks, scene.wide_stack, PT_THREADS)}};
         const Pt<N, T> pt{q, scene, g, Bpt<N, T, 1>{q, scene, g, 0, nullptr, nullptr}};
         Ray<N, T> ray;

@@ -289,7 +289,7 @@ __global__ void __launch_bounds__(WALK_THREADS) walk_mesh_kernel(
                 hit.distance = list.distance[k];
                 hit.kind = static_cast<int>(HitKind::NONE);
                 hit.index = -1;
-                group.template mesh<false>(active, ray, hit.distance, hit.kind, hit.index);
+                group.template mesh<false, false>(active, ray, hit.distance, hit.kind, hit.index);
                 const bool found = active && hit.kind == static_cast<int>(HitKind::FACET);
                 bool recast = false;
                 if (found && scene.flat_shading == 0)

@@ -235,8 +235,9 @@ struct GroupQueries final
                 return threadIdx.x % 32 / WIDE * WIDE;
         }
 
-        // The flat and solid shapes of a query, a shape to a lane: the closest hit before `best`, the first of several at one
-        // distance; (ANY) whether there is one, in `kind`.
+        // The flat and solid shapes of a query, a shape to a lane: the closest
+        // hit before `best`, the first of several at one distance; (ANY) whether
+        // there is one, in `kind`.
         template <bool ANY>
         __device__ void shapes(const bool active, const Ray<N, T>& ray, T& best, int& kind, int& index) const
         {
@@ -291,8 +292,18 @@ struct GroupQueries final
                 }
         }
 
-        // The meshes of a query: the closest hit before `best`, or (ANY) whether there is one, in `kind`.
-        template <bool ANY>
+        // The meshes of a query: the closest hit before `best`, or (ANY) whether
+        // there is one, in `kind`.  ONE: the scene has one mesh at most.
+        //
+        // A mesh's bound is its root box entry (shapes/mesh.cpp:225-229).  Of
+        // several meshes eight bounds are tested at a time, a lane each, and the
+        // groups then visit theirs, each in its own order, together; a bound that
+        // lies behind a hit found in the meantime has no child before it either
+        // (3-space, single precision, 500 meshes: one bound after another, by all
+        // lanes of a group, 23.7 ms per pass, so 11.3; path tracing 23.5 and 10.4).
+        // Scenes of one mesh are 1 to 2 % faster without the rounds, and path
+        // tracing without their code.
+        template <bool ANY, bool ONE>
         __device__ void mesh(const bool active, const Ray<N, T>& ray, T& best, int& kind, int& index) const
         {
                 const DeviceScene<N, T, C>& s = q.s;
@@ -307,49 +318,62 @@ struct GroupQueries final
                                 neg |= 1u << i;
                         }
                 }
-                for (int first = 0; first < s.mesh_count; first += WIDE)
+                if (ONE || s.mesh_count <= 1)
                 {
-                        // a mesh's bound is its root box entry (shapes/mesh.cpp:225-229),
-                        // tested by a lane per mesh: its near side does not depend on
-                        // `best`, with which it is compared when the mesh's turn comes
-                        const int mine = first + static_cast<int>(lane());
-                        T bound = -1;
-                        if (active && !(ANY && kind != static_cast<int>(HitKind::NONE)) && mine < s.mesh_count)
+                        const bool enters = active && s.mesh_count > 0 &&
+                                            !(ANY && kind != static_cast<int>(HitKind::NONE)) &&
+                                            !(box_volume<N>(s.meshes[0].lo, s.meshes[0].hi, ray, best) < 0);
+                        if (__any_sync(FULL, enters))
                         {
-                                bound = box_volume<N>(s.meshes[mine].lo, s.meshes[mine].hi, ray, best);
+                                tree<ANY>(enters, 0, ray, rec, neg, best, kind, index);
                         }
-                        unsigned meshes = (__ballot_sync(FULL, !(bound < 0)) >> group_shift()) & 0xffu;
-                        while (__any_sync(FULL, meshes != 0))
+                        return;
+                }
+                if constexpr (!ONE)
+                {
+                        unsigned entered = 0; // of the eight meshes before `m`, those not yet visited
+                        for (int m = 0;;)
                         {
-                                const int next = meshes != 0 ? __ffs(static_cast<int>(meshes)) - 1 : 0;
-                                const T near = __shfl_sync(FULL, bound, next, WIDE);
-                                int top = 0;
-                                if (meshes != 0 && near <= best)
+                                if (!__any_sync(FULL, entered != 0))
                                 {
-                                        top = 1;
-                                        if (lane() == 0)
+                                        if (m >= s.mesh_count)
                                         {
-                                                stack.near[0] = 0;
-                                                stack.ref[0] = static_cast<std::uint32_t>(first + next);
+                                                return;
                                         }
+                                        const int mine = m + static_cast<int>(lane());
+                                        const bool enters =
+                                                active && mine < s.mesh_count &&
+                                                !(ANY && kind != static_cast<int>(HitKind::NONE)) &&
+                                                !(box_volume<N>(s.meshes[mine].lo, s.meshes[mine].hi, ray, best) < 0);
+                                        entered = (__ballot_sync(FULL, enters) >> group_shift()) & 0xffu;
+                                        m += WIDE;
+                                        continue;
                                 }
-                                meshes &= meshes - 1;
-                                __syncwarp();
-                                traverse<ANY>(ray, rec, neg, best, kind, index, top);
-                                if (ANY && kind != static_cast<int>(HitKind::NONE))
-                                {
-                                        meshes = 0;
-                                }
+                                const int next = __ffs(static_cast<int>(entered)) - 1;
+                                tree<ANY>(entered != 0, static_cast<std::uint32_t>(m - WIDE + next), ray, rec, neg, best,
+                                          kind, index);
+                                entered = ANY && kind != static_cast<int>(HitKind::NONE) ? 0 : entered & (entered - 1);
                         }
                 }
         }
 
 private:
-        // Visits what is stacked and all that follows from it.
+        // The tree of a mesh, whose root is wide node `root`.
         template <bool ANY>
-        __device__ void traverse(const Ray<N, T>& ray, const Vec<N, T>& rec, const unsigned neg, T& best, int& kind,
-                                 int& index, int top) const
+        __device__ __forceinline__ void tree(const bool enters, const std::uint32_t root, const Ray<N, T>& ray,
+                                             const Vec<N, T>& rec, const unsigned neg, T& best, int& kind, int& index) const
         {
+                int top = 0;
+                if (enters)
+                {
+                        top = 1;
+                        if (lane() == 0)
+                        {
+                                stack.near[0] = 0;
+                                stack.ref[0] = root;
+                        }
+                }
+                __syncwarp();
                 while (__any_sync(FULL, top > 0))
                 {
                         bool node = false;
@@ -573,7 +597,24 @@ private:
 // calls them together.  The lanes test the flat and solid shapes; then the
 // rays that may enter a mesh (one in five) go to the warp's four groups, four
 // at a time, through shuffles.
+//
+// MANY: scenes of several meshes, or of so many flat and solid shapes that the
+// groups test those as well.  In the queries of a bounce only part of a warp's
+// lanes have a ray, and they wait for the one whose ray is blocked last; worth
+// the shuffles among more than a hundred shapes (path tracing among 1,000
+// parallelotopes, 3-space single and double precision: 21.2 and 35.9 ms, shared
+// out 12.5 and 21.2; among 100 7.2 and 11.7, shared out 7.1 and 11.3; among 40
+// 4.2 and 7.1, shared out 5.0 and 9.5).  Kernels of their own, since the
+// additional code costs the other scenes 2 to 3 % (3-space double).
+inline constexpr int SHARED_SHAPES = 128;
+
 template <int N, typename T, int C>
+inline bool many_shapes(const DeviceScene<N, T, C>& scene)
+{
+        return scene.mesh_count > 1 || scene.flat_count + scene.solid_count >= SHARED_SHAPES;
+}
+
+template <int N, typename T, int C, bool MANY>
 struct WarpQueries final
 {
         static constexpr unsigned FULL = 0xffffffffu;
@@ -581,19 +622,26 @@ struct WarpQueries final
         const SceneQueries<N, T, C>& q;
         const GroupQueries<N, T, C> group;
 
-        struct MeshHit final
+        struct GroupHit final
         {
                 T distance;
                 int kind;
                 int index;
         };
 
-        // the meshes of the lanes that want them: the closest hit before
-        // `best` (ANY: whether there is one), kind NONE without
-        template <bool ANY>
-        NBPT_CALL MeshHit mesh(const bool wants, const Ray<N, T>& ray, const T best) const
+        // whether the groups test the flat and solid shapes
+        __device__ bool share_shapes() const
         {
-                MeshHit mine{best, static_cast<int>(HitKind::NONE), -1};
+                return MANY && q.s.flat_count + q.s.solid_count >= SHARED_SHAPES;
+        }
+
+        // the meshes, and the flat and solid shapes that are shared out, of the
+        // lanes that want them: the closest hit before `best` (ANY: whether there
+        // is one), kind NONE without
+        template <bool ANY>
+        NBPT_CALL GroupHit shared(const bool wants, const Ray<N, T>& ray, const T best) const
+        {
+                GroupHit mine{best, static_cast<int>(HitKind::NONE), -1};
                 const int lane = static_cast<int>(threadIdx.x & 31);
                 const int my_group = lane / WIDE;
                 unsigned pending = __ballot_sync(FULL, wants);
@@ -617,7 +665,11 @@ struct WarpQueries final
                         T distance = __shfl_sync(FULL, best, from);
                         int kind = static_cast<int>(HitKind::NONE);
                         int index = -1;
-                        group.template mesh<ANY>(active, r, distance, kind, index);
+                        if (share_shapes())
+                        {
+                                group.template shapes<ANY>(active, r, distance, kind, index);
+                        }
+                        group.template mesh<ANY, !MANY>(active, r, distance, kind, index);
                         // back to the ray's lane
                         const int place = __popc(pending & ((1u << lane) - 1));
                         const int to = (place % (32 / WIDE)) * WIDE;
@@ -648,10 +700,14 @@ struct WarpQueries final
                 if (active)
                 {
                         ++q.counters.queries;
-                        q.closest_shape(ray, h.distance, h.kind, h.index);
-                        wants = q.enters_mesh(ray, h.distance);
+                        wants = share_shapes();
+                        if (!wants)
+                        {
+                                q.closest_shape(ray, h.distance, h.kind, h.index);
+                                wants = q.enters_mesh(ray, h.distance);
+                        }
                 }
-                const MeshHit m = mesh<false>(wants, ray, h.distance);
+                const GroupHit m = shared<false>(wants, ray, h.distance);
                 if (m.kind != static_cast<int>(HitKind::NONE))
                 {
                         h.distance = m.distance;
@@ -673,10 +729,14 @@ struct WarpQueries final
                 if (active)
                 {
                         ++q.counters.queries;
-                        hit = q.any_shape(ray, max_distance);
-                        wants = !hit && q.enters_mesh(ray, max_distance);
+                        wants = share_shapes();
+                        if (!wants)
+                        {
+                                hit = q.any_shape(ray, max_distance);
+                                wants = !hit && q.enters_mesh(ray, max_distance);
+                        }
                 }
-                const MeshHit m = mesh<true>(wants, ray, max_distance);
+                const GroupHit m = shared<true>(wants, ray, max_distance);
                 return hit || m.kind != static_cast<int>(HitKind::NONE);
         }
 
