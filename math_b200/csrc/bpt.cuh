@@ -776,6 +776,7 @@ struct Bpt final
                 return sight;
         }
 
+        // The strategies of s = 0 and s >= 2.
         __device__ __forceinline__ Sight connect_strategy(const int s_count, const int t_count, Color<C>& out)
         {
                 HeldVertex cv = camera[t_count - 1];
@@ -812,17 +813,6 @@ struct Bpt final
                 {
                         return Sight::BLOCKED;
                 }
-                if (s_count == 1)
-                {
-                        int li;
-                        ArriveSample<N, T, C> as;
-                        if (!light_arrival(t_count, li, as))
-                        {
-                                return Sight::BLOCKED;
-                        }
-                        return connect_light(t_count, li, as, out);
-                }
-
                 HeldVertex lv = light[s_count - 1];
                 // compute_color (connect.cpp:187-221)
                 const Vec<N, T> v = lv.pos - cv.pos;

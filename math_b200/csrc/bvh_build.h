@@ -20,11 +20,12 @@ namespace nbpt::host
 inline constexpr double BOX_R_RATE = 2.4e9;
 inline constexpr double SIMPLEX_RATE = 0.8e9;
 
-// Entries of the traversal stack (the reference's BvhStack holds 64,
-// src/geometry/accelerators/bvh_stack.h:26).  Depth-first traversal keeps at
-// most one entry per interior node above the current node, so a tree whose
-// leaves are at most this deep (root at depth 0) never overflows it; both
-// builders refuse deeper trees, which only degenerate meshes produce.
+// The deepest tree that a mesh may have (leaves, the root at depth 0): the
+// reference's traversal stack holds 64 entries
+// (src/geometry/accelerators/bvh_stack.h:26), at most one per interior node
+// above the current one.  Both builders refuse deeper trees, which only
+// degenerate meshes produce; the queries' stacks are as deep as a scene's
+// trees need (wide_bvh.cuh).
 inline constexpr int BVH_MAX_DEPTH = 64;
 
 template <int N, typename T>

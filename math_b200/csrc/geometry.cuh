@@ -336,37 +336,9 @@ struct Simplex final
                 return true;
         }
 
-        // Hit distance, or 0 for no hit (a hit has t > 0).
+        // Hit distance, or 0 for no hit (a hit has t > 0).  Without branches: every
+        // plane is loaded at once, where branches would make the loads a chain.
         NBPT_HD T intersect(const Ray<N, T>& r) const
-        {
-                const T t = plane.intersect(r);
-                if (!(t > 0))
-                {
-                        return 0;
-                }
-                const Vec<N, T> p = r.point(t);
-                T bc[N - 1];
-#pragma unroll
-                for (int i = 0; i < N - 1; ++i)
-                {
-                        bc[i] = planes[i].distance(p);
-                        if (!(bc[i] > 0 && bc[i] < 1))
-                        {
-                                return 0;
-                        }
-                }
-                T sum = bc[0];
-#pragma unroll
-                for (int i = 1; i < N - 1; ++i)
-                {
-                        sum += bc[i];
-                }
-                return (sum < 1) ? t : T(0);
-        }
-
-        // intersect() without branches: every plane is loaded at once, where
-        // branches would make the loads a chain.
-        NBPT_HD T intersect_whole(const Ray<N, T>& r) const
         {
                 const T t = plane.intersect(r);
                 const Vec<N, T> p = r.point(t);
@@ -598,36 +570,6 @@ struct SolidParallelotope final
 
 // ---------------------------------------------------------------------------
 // axis-aligned box tests (src/geometry/spatial/bounding_box.h:121-194)
-
-// Traversal test with the precomputed reciprocal direction and signs.
-template <int N, typename T>
-NBPT_HD bool box_hit(
-        const T* lo,
-        const T* hi,
-        const Vec<N, T>& org,
-        const Vec<N, T>& rec,
-        const unsigned neg_mask,
-        const T max_distance)
-{
-        T near = 0;
-        T far = max_distance;
-#pragma unroll
-        for (int i = 0; i < N; ++i)
-        {
-                const bool negative = (neg_mask >> i) & 1u;
-                const T d = org[i];
-                const T r = rec[i];
-                const T a1 = ((negative ? hi[i] : lo[i]) - d) * r;
-                const T a2 = ((negative ? lo[i] : hi[i]) - d) * r;
-                near = a1 > near ? a1 : near;
-                far = a2 < far ? a2 : far;
-                if (far < near)
-                {
-                        return false;
-                }
-        }
-        return true;
-}
 
 // Volume test: entry distance (0 from inside) or -1 for no hit.
 template <int N, typename T>

@@ -2036,9 +2036,6 @@ public:
                                 rec.lo[d] = root.lo[d];
                                 rec.hi[d] = root.hi[d];
                         }
-                        rec.node_offset = m.node_offset;
-                        rec.index_offset = m.index_offset;
-                        rec.facet_offset = m.facet_offset;
                         mesh_records_.push_back(rec);
                 }
                 mesh_nodes.clear();
@@ -2146,8 +2143,6 @@ public:
                 device_.solid_count = static_cast<int>(solid_.size());
                 device_.meshes = d_meshes_.get();
                 device_.mesh_count = static_cast<int>(mesh_records_.size());
-                device_.nodes = d_nodes_.get();
-                device_.indices = d_indices_.get();
                 device_.wide = d_wide_.get();
                 device_.leaf_facets = d_leaf_facets_.get();
                 device_.wide_stack = wide_stack_;
@@ -2203,8 +2198,6 @@ public:
                         device_1_.solid_count = device_.solid_count;
                         device_1_.meshes = device_.meshes;
                         device_1_.mesh_count = device_.mesh_count;
-                        device_1_.nodes = device_.nodes;
-                        device_1_.indices = device_.indices;
                         device_1_.wide = device_.wide;
                         device_1_.leaf_facets = device_.leaf_facets;
                         device_1_.wide_stack = device_.wide_stack;

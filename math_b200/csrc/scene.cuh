@@ -4,12 +4,9 @@
 //   flat[]      flat (n-1)-parallelotopes (walls, light carriers): hyperplane,
 //               N-1 slab planes, bounding box, material, attached light
 //   solid[]     solid n-parallelotopes: N slabs, bounding box, material
-//   meshes[]    one record per mesh shape: root box, node/index/facet offsets
-//   nodes[]     binary BVH nodes in depth-first order, as the reference lays
-//               them out (src/geometry/accelerators/bvh.h:49-62, bvh.cpp:35-67):
-//               box, second-child or first-object offset, object count, axis
-//   indices[]   facet index per leaf slot
-//   wide[]      the same tree with eight children to a node (wide_bvh.cuh)
+//   meshes[]    one record per mesh shape: root box
+//   wide[]      BVH nodes of eight children (wide_bvh.cuh), from the binary
+//               nodes (BvhNode), which the scene keeps for export
 //   leaf_facets[] the simplex of every leaf slot
 //   facets[]    (n-1)-simplex records (hyperplane + N-1 barycentric planes),
 //               material and vertex-normal indices
@@ -111,9 +108,6 @@ struct MeshShape final
 {
         T lo[N];
         T hi[N];
-        int node_offset;
-        int index_offset;
-        int facet_offset;
 };
 
 template <typename T, int C>
@@ -193,8 +187,6 @@ struct DeviceScene final
         int solid_count;
         const MeshShape<N, T>* meshes;
         int mesh_count;
-        const BvhNode<N, T>* nodes;
-        const std::uint32_t* indices;
         const WideChild<N, T>* wide; // the root of mesh m is wide node m
         const LeafFacet<N, T>* leaf_facets;
         int wide_stack; // stack entries of a query (wide_stack_entries)

@@ -635,19 +635,12 @@ NBPT_HD BrdfSample<N, C, T> brdf_sample(
         return s;
 }
 
-// brdf_sample() and brdf_pdf() out of line, like brdf_terms_call().
+// brdf_sample() out of line, like brdf_terms_call().
 template <int N, int C, typename T>
 NBPT_HD_CALL BrdfSample<N, C, T> brdf_sample_call(Pcg& g, const ShadingConstants<T>& sc, const T roughness,
                                                   const Color<C>& f0, const Color<C>& rho_ss, const Vec<N, T>& n,
                                                   const Vec<N, T>& v, BrdfTerms* const terms)
 {
         return brdf_sample<N, C, true>(g, sc, roughness, f0, rho_ss, n, v, terms);
-}
-
-template <int N, typename T>
-NBPT_HD_CALL T brdf_pdf_call(const ShadingConstants<T>& sc, const T roughness, const Vec<N, T>& n, const Vec<N, T>& v,
-                             const Vec<N, T>& l)
-{
-        return brdf_pdf<N>(sc, roughness, n, v, l);
 }
 } // namespace nbpt

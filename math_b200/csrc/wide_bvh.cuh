@@ -487,7 +487,7 @@ private:
         {
                 ++q.counters.facets;
                 const LeafFacet<N, T> f = q.s.leaf_facets[slot];
-                const T t = f.simplex.intersect_whole(ray);
+                const T t = f.simplex.intersect(ray);
                 facet = f.facet;
                 return t > 0 && t < best ? t : infinity<T>();
         }
@@ -572,7 +572,7 @@ private:
                 }
         }
 
-        // near and far of the slab test (box_hit): a NaN product, of a zero
+        // near and far of the slab test: a NaN product, of a zero
         // distance and an infinite reciprocal, changes neither
         __device__ static float slab_max(const float near, const float a)
         {
