@@ -187,17 +187,6 @@ __global__ void sj_points_kernel(
         }
 }
 
-// Blocks of 128 threads per SM of the kernels over the strategies: the
-// registers of paths_light_kernel (65536 / (128 * blocks)) and the grid that
-// paths_connect_kernel strides over its queues.  Where these kernels' shape
-// hardly matters the figures of the earlier persistent kernels stand: 16 in
-// single precision, 8 in double (12 in 3-space).
-template <int N, typename T>
-struct PathsMinBlocks final
-{
-        static constexpr int value = std::is_same_v<T, double> ? (N == 3 ? 12 : 8) : 16;
-};
-
 // ---------------------------------------------------------------------------
 // Paths: one per pixel sample, with the random stream seed_seq{seed, pass,
 // p, i + 1}.  A chunk of pixels runs through these kernels:
@@ -443,7 +432,11 @@ __device__ inline Bpt<N, T, 1, true> connection(const SceneQueries<N, T, 1>& q, 
         return bpt;
 }
 
+// The grid that strides over the queues: 4 to 64 blocks per SM take the same
+// time within 3 % but for a small double-precision job, whose queues 4 and 64
+// take 15 % longer (5-space, 0.19 ms with 8 to 32).
 inline constexpr int CONNECT_THREADS = 128;
+inline constexpr int CONNECT_BLOCKS_PER_SM = 16;
 
 // One thread per queued strategy (the grid strides over the queues): its
 // contribution factors and its line of sight past the flat and solid shapes.
@@ -677,9 +670,11 @@ __global__ void __launch_bounds__(CONNECT_THREADS) connect_sight_kernel(
 // One thread per path: the light samples of the s = 1 strategies, drawn in
 // t order from the path's stream where the light subpath left it; each
 // usable sample is kept and its strategy queued for the connect kernel, with
-// the path's s = 0 and s >= 2 strategies.
+// the path's s = 0 and s >= 2 strategies.  As many registers as it takes: capped
+// for more resident blocks (16 of single precision, 12 or 8 of double) it took
+// 6 to 12 % longer (3-space double 178 -> 200 us, 5-space single 223 -> 250).
 template <int N, typename T>
-__global__ void __launch_bounds__(128, (PathsMinBlocks<N, T>::value)) paths_light_kernel(
+__global__ void __launch_bounds__(128) paths_light_kernel(
         const DeviceScene<N, T, 1> scene,
         const long long paths,
         const int max_depth,

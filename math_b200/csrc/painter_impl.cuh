@@ -2882,7 +2882,7 @@ public:
                         task_count_.allocate(5);
                         walk_counters_.allocate(1);
                         walk_blocks_ = sms * WALK_BLOCKS_PER_SM;
-                        connect_blocks_ = sms * PathsMinBlocks<N, T>::value;
+                        connect_blocks_ = sms * CONNECT_BLOCKS_PER_SM;
                 }
 
                 NBPT_CUDA(cudaEventCreate(&ev_start_));
@@ -3165,7 +3165,7 @@ public:
                                                 scene_1, n, max_depth_, vertices_.get(), rng_.get(), tape_.get(), tape_words_,
                                                 arrivals_.get(), queues, cancel_.get());
                                         NBPT_CUDA(cudaGetLastError());
-                                        connect_kernel()<<<connect_blocks_, 128, 0, stream_>>>(
+                                        connect_kernel()<<<connect_blocks_, CONNECT_THREADS, 0, stream_>>>(
                                                 scene_1, max_depth_, vertices_.get(), tape_.get(), tape_words_, arrivals_.get(),
                                                 queues, sights, stats_.get());
                                         NBPT_CUDA(cudaGetLastError());
