@@ -64,8 +64,10 @@ typedef struct nbpt_statistics
         long long ray_count;    /* scene queries of the last pass */
         long long sample_count; /* paths of the last pass (actual samples) */
         double previous_pass_duration; /* seconds, device time of the last pass */
-        double paths_seconds;          /* device time of the path kernel, last pass */
-        unsigned long long nodes;      /* BVH nodes visited, last pass */
+        double paths_seconds;          /* device time of the path kernels, last pass */
+        /* BVH boxes tested, last pass: the children of the eight-child nodes
+         * visited */
+        unsigned long long nodes;
         unsigned long long facets;     /* facet records tested, last pass */
         unsigned long long shapes;     /* other shapes tested, last pass */
         long long kernel_launches;     /* kernels launched by the last pass */
@@ -242,9 +244,9 @@ typedef struct nbpt_painter_options
         int slab_end;
         int pixel_sums; /* NBPT_PIXEL_SUMS_* */
         /* device bytes of the per-chunk path buffers (0: a tenth of the
-         * device's memory within [4, 16] GiB); a pass runs its paths in
-         * chunks of as many as they hold, with the same images whatever the
-         * size */
+         * device's memory within [4, 16] GiB; at most a fifth of it within
+         * [4, 32] GiB); a pass runs its paths in chunks of as many as they
+         * hold, with the same images whatever the size */
         long long chunk_budget;
 } nbpt_painter_options;
 nbpt_painter* nbpt_painter_create_options(nbpt_scene* scene, const nbpt_painter_options* options);
@@ -364,10 +366,11 @@ int nbpt_server_job(nbpt_server* server, long long job, nbpt_job_info* info);
 /* Device bytes of per-chunk path buffers for each render the server creates
  * from now on (renders already submitted keep theirs); 0 restores the
  * default, an equal share of the memory budget per job slot and at least
- * 4 GiB.  A pass's paths run in chunks of as many paths as these buffers
- * hold, and each chunk ends in a tail where the persistent path kernels run
- * out of paths; larger chunks shorten the tails, while fewer renders fit in
- * the memory budget at once.  math_b200.tuning picks it by measurement.
+ * 4 GiB, of which a render takes what it would take alone.  A pass's paths
+ * run in chunks of as many paths as these buffers hold, a chunk in some forty
+ * launches that each end with their longest rays; larger chunks have fewer of
+ * them, while fewer renders fit in the memory budget at once.
+ * math_b200.tuning picks it by measurement.
  * No reference counterpart: the reference's painter keeps one path per
  * thread (src/painter/painting/painting.cpp:181-206). */
 int nbpt_server_set_chunk_budget(nbpt_server* server, long long bytes);
@@ -463,8 +466,8 @@ int nbpt_test_pcg(const unsigned* seed, int seed_words, int count, unsigned* out
 int nbpt_test_canonical(const unsigned* seed, int seed_words, int count, int use_double, double* out);
 /* the host BVH build alone (no GPU needed): node count and the depth of the
  * deepest leaf of the facet BVH of a mesh (vertices [vertex_count][dimension],
- * facets [facet_count][dimension]); NBPT_ERROR when the tree is deeper than the
- * traversal stack (64 entries, the reference's BvhStack:
+ * facets [facet_count][dimension]); NBPT_ERROR when the tree is deeper than 64
+ * (the entries of the reference's traversal stack,
  * src/geometry/accelerators/bvh_stack.h:26), as nbpt_scene_finalize reports */
 int nbpt_test_bvh_build(int dimension, int precision, const double* vertices, long long vertex_count,
                         const int* facets, long long facet_count, long long* nodes, int* depth);

@@ -5,6 +5,8 @@
 
 #include <cuda_runtime.h>
 
+#include <algorithm>
+#include <atomic>
 #include <iterator>
 #include <map>
 #include <unordered_map>
@@ -172,5 +174,39 @@ std::size_t cached()
         Cache& c = cache();
         const std::lock_guard lock(c.mutex);
         return c.bytes;
+}
+
+namespace
+{
+// total / `divisor` of the current device's memory, within [4 GiB, `most`]
+long long memory_share(const std::size_t divisor, const long long most)
+{
+        constexpr long long LEAST = 4LL << 30;
+        static std::atomic<std::size_t> total_by_device[64] = {};
+        int device = 0;
+        if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= 64)
+        {
+                cudaGetLastError();
+                return LEAST;
+        }
+        std::size_t total = total_by_device[device].load();
+        if (total == 0)
+        {
+                std::size_t free = 0;
+                cuda_check(cudaMemGetInfo(&free, &total), "cudaMemGetInfo");
+                total_by_device[device] = total;
+        }
+        return std::min(most, std::max(LEAST, static_cast<long long>(total / divisor)));
+}
+} // namespace
+
+long long chunk_budget()
+{
+        return memory_share(10, 16LL << 30);
+}
+
+long long largest_chunk_budget()
+{
+        return memory_share(5, 32LL << 30);
 }
 } // namespace nbpt::pool

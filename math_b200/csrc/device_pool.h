@@ -24,4 +24,9 @@ void release(void* p, std::size_t bytes, int device);
 std::size_t trim();
 // bytes held in the cache
 std::size_t cached();
+// Bytes of the current device's memory that one render's per-chunk path
+// buffers take: by themselves, a tenth within [4, 16] GiB, and at most, when
+// the caller asks for more, a fifth within [4, 32] GiB.
+long long chunk_budget();
+long long largest_chunk_budget();
 } // namespace nbpt::pool

@@ -15,8 +15,8 @@ struct Statistics final
         long long ray_count;
         long long sample_count;
         double previous_pass_duration; // seconds, device time of the last pass
-        double paths_seconds;          // device time of the path kernel, last pass
-        unsigned long long nodes;      // BVH nodes visited, last pass
+        double paths_seconds;          // device time of the path kernels, last pass
+        unsigned long long nodes;      // BVH boxes tested (children of wide nodes), last pass
         unsigned long long facets;     // facet records tested, last pass
         unsigned long long shapes;     // other shapes tested, last pass
         long long kernel_launches;     // kernels launched by the last pass
@@ -131,8 +131,8 @@ public:
                                                         long long chunk_budget = 0, int pixel_sums = 0) = 0;
         // device bytes create_painter would allocate.  chunk_budget: bytes
         // for the buffers of one chunk of paths (0: a tenth of the device's
-        // memory within [4, 16] GiB); the job server gives each of its slots
-        // a share of its memory budget
+        // memory within [4, 16] GiB; at most a fifth within [4, 32] GiB); the
+        // job server gives each of its slots a share of its memory budget
         virtual long long painter_bytes(int samples_per_pixel, int max_depth,
                                         Integrator integrator = Integrator::BPT,
                                         long long chunk_budget = 0, int pixel_sums = 0) const = 0;

@@ -2540,7 +2540,7 @@ class PainterT final : public Painter
 {
         const SceneT<N, T, C>* scene_;
         bool flat_shading_;
-        long long chunk_budget_; // bytes for the chunk buffers, 0: chunk_budget()
+        long long chunk_budget_; // bytes for the chunk buffers, 0: pool::chunk_budget()
         int spp_request_;
         int spp_;
         int strata_;
@@ -2638,41 +2638,6 @@ class PainterT final : public Painter
         int launches_accumulate_ = 0;
         Statistics statistics_{};
 
-        // Device memory for the per-path buffers of one chunk.  A chunk's waves
-        // end with the longest rays of each on an emptying GPU, and every chunk
-        // has some forty launches; larger chunks have fewer of both per path.
-        // Milliseconds of a pass with 4 / 8 / 16 / 32 GiB: 4-space spectral f32
-        // (7.1 M paths) 50.2 / 45.3 / 42.7 / 41.3, 5-space f32 (1.7 M, depth 8)
-        // 21.3 / 16.8 / 13.0 / 12.9, 4-space sphere f32 8.4 / 7.9 / 7.4 / 7.4,
-        // 3-space f64 6.3 / 6.2 / 6.2 / 6.2.  A tenth of the device's memory,
-        // within [4, 16] GiB: twice that gains at most 3 % and doubles what a
-        // first render has to allocate, which takes up to 0.4 s for 32 GiB
-        // (NBPT_CHUNK_BUDGET_GB, when defined, sets it for sweeps).
-        static long long chunk_budget()
-        {
-#ifdef NBPT_CHUNK_BUDGET_GB
-                return static_cast<long long>(NBPT_CHUNK_BUDGET_GB) << 30;
-#else
-                static std::atomic<long long> by_device[64] = {};
-                int device = 0;
-                if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= 64)
-                {
-                        cudaGetLastError();
-                        return 4LL << 30;
-                }
-                long long b = by_device[device].load();
-                if (b == 0)
-                {
-                        std::size_t free = 0;
-                        std::size_t total = 0;
-                        NBPT_CUDA(cudaMemGetInfo(&free, &total));
-                        b = std::min(16LL << 30, std::max(4LL << 30, static_cast<long long>(total / 10)));
-                        by_device[device] = b;
-                }
-                return b;
-#endif
-        }
-
         // The strategy queues of a chunk (the tasks, then the lines of sight
         // left to the meshes), in whose place the walks keep their lists and
         // queues before there are strategies.
@@ -2695,7 +2660,17 @@ class PainterT final : public Painter
         // 32-bit path counter
         static constexpr long long PT_CHUNK_PATHS = 1LL << 30;
 
-        // budget: bytes for the chunk buffers, 0 for chunk_budget()
+        // Pixels of a chunk.  budget: bytes for its buffers, at most
+        // pool::largest_chunk_budget(); 0: pool::chunk_budget().
+        //
+        // A chunk's waves end with the longest rays of each on an emptying GPU, and
+        // every chunk has some forty launches; larger chunks have fewer of both per
+        // path.  Milliseconds of a pass with 4 / 8 / 16 / 32 GiB: 4-space spectral
+        // f32 (7.1 M paths) 50.2 / 45.3 / 42.7 / 41.3, 5-space f32 (1.7 M, depth 8)
+        // 21.3 / 16.8 / 13.0 / 12.9, 4-space sphere f32 8.4 / 7.9 / 7.4 / 7.4,
+        // 3-space f64 6.3 / 6.2 / 6.2 / 6.2.  Unless the caller asks for more, 16
+        // GiB: twice that gains at most 3 % and doubles what a first render has to
+        // allocate, which takes up to 0.4 s for 32 GiB.
         static long long chunk_pixels(const long long pixels, const int spp, const int max_depth,
                                       const Integrator integrator, const long long budget = 0)
         {
@@ -2704,7 +2679,7 @@ class PainterT final : public Painter
                         return std::max(1LL, std::min(pixels, PT_CHUNK_PATHS / spp));
                 }
                 const long long per_pixel = chunk_path_bytes(max_depth) * spp;
-                const long long b = budget > 0 ? std::min(budget, chunk_budget()) : chunk_budget();
+                const long long b = budget > 0 ? std::min(budget, pool::largest_chunk_budget()) : pool::chunk_budget();
                 long long c = std::max(1LL, std::min(pixels, b / per_pixel));
                 return std::min(c, (TASK_MAX_PATHS - 1) / spp);
         }

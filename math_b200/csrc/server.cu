@@ -2,7 +2,7 @@
 #include "server.h"
 
 #include "cuda_error.h"
-
+#include "device_pool.h"
 
 #include <cuda_runtime.h>
 
@@ -213,7 +213,7 @@ long long Server::submit_render(Scene* const scene, const int spp, const int max
         job->info.passes_done = 0;
         {
                 const std::lock_guard lock(mutex_);
-                job->chunk_budget = slot_chunk_budget();
+                job->chunk_budget = chunk_budget_ > 0 ? chunk_budget_ : std::min(slot_chunk_budget(), pool::chunk_budget());
         }
         job->info.footprint =
                 scene->painter_bytes(spp, max_depth, Integrator::BPT, job->chunk_budget) + scene->device_bytes();

@@ -83,9 +83,10 @@ public:
         void hold_admission(bool hold);
         // device bytes of chunk buffers (the per-chunk path buffers of the
         // BPT kernels) of each render the server creates from now on; 0: an
-        // equal share of the memory budget per slot, at least 4 GiB.  Larger
-        // chunks leave less of each pass to the persistent kernels' tails;
-        // fewer renders then fit in the budget at once.
+        // equal share of the memory budget per slot, at least 4 GiB, of which
+        // a render takes what it would take alone (pool::chunk_budget).  Larger
+        // chunks are fewer, each of some forty launches that end with their
+        // longest rays; fewer renders then fit in the budget at once.
         void set_chunk_budget(long long bytes);
         long long chunk_budget() const;
         double now() const;

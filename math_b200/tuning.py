@@ -2,12 +2,11 @@
 
 A render's pass runs its paths in chunks of as many paths as its chunk
 buffers hold (vertices, random-stream states, tapes and strategy queues:
-about 6 KB per path at depth 8), and every chunk ends in a tail where the
-persistent path kernels run out of paths and their blocks drain one lane at
-a time.  With many renders on the GPU at once, each render's chunk budget is
-a share of the server's memory budget: small shares mean short chunks and
-long tails, large shares mean fewer renders at once to fill each other's
-tails.  Which balance is best depends on the workload's mix of scene sizes,
+about 6 KB per path at depth 8), and every chunk is some forty launches that
+each end with their longest rays on an emptying GPU.  With many renders on the
+GPU at once, each render's chunk budget is a share of the server's memory
+budget: small shares mean short chunks and many such ends, large shares mean
+fewer renders at once to fill each other's.  Which balance is best depends on the workload's mix of scene sizes,
 so it is measured: `tune_chunk_budget` runs the caller's workload once per
 candidate budget and keeps the fastest, and returns every trial for the log.
 """
