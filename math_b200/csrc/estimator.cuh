@@ -17,7 +17,7 @@
 // partial_sort perform, sources are merged into a receiving pixel in
 // increasing pixel index, and all sums are in float as the reference keeps
 // them.  From the same samples the image is therefore the reference's, bit
-// for bit.  Every receiving pixel is gathered by its own thread or warp, so
+// for bit.  Every receiving pixel's groups are merged by one thread or warp, so
 // no atomics are needed.
 //
 // The same merges run with the radiance and weight sums in double (the sum
@@ -97,7 +97,7 @@ struct ColorGroup final
 };
 
 // create_with_sum (samples/com/create.h:28-55): the sums of a group of more
-// than HELD_OUT samples, without those held out, in order.  Four samples'
+// than HELD_OUT samples, without those held out, in order.  Eight samples'
 // colours are loaded before the first is added, since each is a load whose
 // address another load gives (64 channels, 27 groups of 27 samples per pixel:
 // with the merges as selections (FullMerge) 12.5 -> 10.3 ms for
@@ -877,7 +877,7 @@ __global__ void __launch_bounds__(128) accumulate_kernel(
 // threads of a block share a few sources: a source's factors (three offsets
 // per sample and axis) are computed once into shared memory, and a warp's
 // lanes read the same samples of the same source.  A group travels as a
-// sample set (120-152 bytes).  Those 4,096 pixels now take 0.15 ms to form
+// sample set (132-152 bytes).  Those 4,096 pixels now take 0.15 ms to form
 // and 0.27 ms to merge, 105,000 of 16 samples 1.2 and 1.4 ms (4.5 before).
 
 // threads of a group_kernel block and the source pixels they share

@@ -1,6 +1,6 @@
 // CUDA kernels of the painter: facet setup, stratified sub-pixel samples,
-// the path kernel, the filtered trimmed accumulation and image resolve, and
-// ray-query and per-function kernels used for verification.
+// BPT's strategies (walk.cuh has the walks before them) and the replay of the
+// colours.
 #pragma once
 
 #include "bpt.cuh"
@@ -214,7 +214,7 @@ struct PathStats final
         unsigned long long nodes;
         unsigned long long facets;
         unsigned long long shapes;
-        unsigned long long overflows; // ray queries ended on a full traversal stack (an error)
+        unsigned long long overflows; // ray queries ended on a full stack (an error)
         unsigned long long nonfinite; // samples whose colour has a NaN or infinite channel
 };
 
@@ -766,8 +766,8 @@ __global__ void __launch_bounds__(128) paths_light_kernel(
 
 // Colours from the tapes: LANES threads per path (32: one warp per path,
 // lane l forms channels l, l + 32, ...; 1: one thread per path).  Every
-// channel goes through the float operations of Bpt::walk, light_path and
-// connect_strategy in the recorded order, the strategies summed in the
+// channel goes through the float operations of Bpt::walk_step, light_start,
+// connect_light and connect_strategy in the recorded order, the strategies summed in the
 // reference's (t, s) order; then the luminance by the reference's
 // left-to-right dot product.
 template <int N, typename T, int C, int LANES>
@@ -868,7 +868,7 @@ __global__ void __launch_bounds__(128) paths_replay_kernel(
                 }
                 else
                 {
-                        break; // not a bounce record: tapes are written by paths_walk_kernel only
+                        break; // not a bounce record: the walk kernels write no other
                 }
         }
         for (int t_count = 2; t_count <= camera_size; ++t_count)

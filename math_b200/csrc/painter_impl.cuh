@@ -4,11 +4,13 @@
 // Scene preparation (host): shapes, meshes, lights and the projector are
 // turned into the device records of scene.cuh with the reference's
 // arithmetic (src/painter/shapes/*.cpp, lights/*.cpp, projectors/*.cpp,
-// shapes/mesh/data.cpp); the mesh BVH is built on the host (bvh_build.cpp)
-// and the facet records in double precision on the GPU (facet_setup_kernel).
+// shapes/mesh/data.cpp); the mesh BVHs are built on the GPU (bvh_device.cuh;
+// on request on the host, bvh_build.cpp), and so are their wide nodes
+// (wide_bvh.cuh) and the facet records, in double precision
+// (facet_setup_kernel).
 //
 // Painter: one pass renders every pixel's stratified samples through the path
-// kernel and folds them into the per-pixel estimator on the device.
+// kernels and folds them into the per-pixel estimator on the device.
 #pragma once
 
 #include "bvh_build.h"
@@ -2697,9 +2699,12 @@ public:
         }
 
         // The scratch of accumulate_groups(): all receiving pixels of most
-        // renders, and for a larger screen ranges long enough that the sources
-        // that two ranges share are few (5-space: 43,000 pixels, of which a
-        // range shares those of its first and last rows).
+        // renders, and ranges of a larger screen.  The launch for a range goes
+        // over all sources from one stride of the last axis before it to one after
+        // it; where that stride exceeds the range, most of them reach no pixel of
+        // it and only their factors are formed (5-space, 43,000 to 50,000 pixels
+        // per range: 25 us per 1,000 pixels x 16 samples on screens of 40^4 and
+        // 50^4, 22 on 18^4).
         static constexpr long long GROUP_BYTES = 512LL << 20;
 
         template <typename S>

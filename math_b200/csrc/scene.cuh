@@ -237,15 +237,15 @@ struct Normals final
         Vec<N, T> shading;
 };
 
-// Statistics counted per query for the roofline: BVH nodes visited, facet
-// records tested and other shapes tested.
+// Statistics counted per query for the roofline: BVH boxes (children of wide
+// nodes), facet records and other shapes tested.
 struct QueryCounters final
 {
         std::uint32_t queries;
         std::uint32_t nodes;
         std::uint32_t facets;
         std::uint32_t shapes;
-        std::uint32_t overflows; // queries that ended on a full traversal stack
+        std::uint32_t overflows; // queries that ended on a full stack
 };
 
 template <int N, typename T, int C>

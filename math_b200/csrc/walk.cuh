@@ -24,7 +24,7 @@
 // of one bounce only, each kernel's code is small, the few rays that reach a
 // BVH (one in five) are gathered into full warps of their own, and a list is
 // read and written in order.  What it costs is the rays' state through
-// memory once per bounce: 72 bytes per ray in 4-space single precision.
+// memory once per bounce: 68 bytes per ray in 4-space single precision.
 #pragma once
 
 #include "kernels.cuh"

@@ -2,7 +2,7 @@
 
 A render's pass runs its paths in chunks of as many paths as its chunk
 buffers hold (vertices, random-stream states, tapes and strategy queues:
-about 6 KB per path at depth 8), and every chunk is some forty launches that
+several KB per path), and every chunk is some forty launches that
 each end with their longest rays on an emptying GPU.  With many renders on the
 GPU at once, each render's chunk budget is a share of the server's memory
 budget: small shares mean short chunks and many such ends, large shares mean
