@@ -1334,6 +1334,10 @@ __global__ void __launch_bounds__(128) accumulate_warp_kernel(
         constexpr int K = C / 32;
         constexpr int WARPS = 4;
         __shared__ float s_weight[WARPS][MAX_GROUP];
+        // the keys of a group's order, which one lane compares (multiplied at each
+        // comparison: 10 % longer with 64 or 81 samples, 5-space 5.13 -> 5.69 ms
+        // for 10,000 pixels)
+        __shared__ float s_contribution[WARPS][MAX_GROUP];
         __shared__ int s_kind[WARPS][MAX_GROUP]; // 0 none, 1 colour, 2 background
         __shared__ int s_order[WARPS][MAX_GROUP];
         __shared__ float s_background[WARPS][MAX_GROUP];
@@ -1435,6 +1439,7 @@ __global__ void __launch_bounds__(128) accumulate_warp_kernel(
                                 const float wf = static_cast<float>(weight);
                                 w[j] = wf;
                                 k = valid[sidx] ? 1 : 2;
+                                s_contribution[warp][j] = wf * lum[sidx];
                         }
                         kind[j] = k;
                 }
@@ -1455,7 +1460,7 @@ __global__ void __launch_bounds__(128) accumulate_warp_kernel(
                                 }
                         }
                         const float* const source_lum = lum + (p - screen.source_first) * spp;
-                        order_group(order, nc, [&](const int i) { return w[i] * source_lum[i]; });
+                        order_group(order, nc, [&](const int i) { return s_contribution[warp][i]; });
                         if (nbg > 1)
                         {
                                 // background samples are ordered by value; reuse
