@@ -96,15 +96,6 @@ public:
                 }
         }
 
-        // keeps a buffer that is large enough
-        void allocate_if_smaller(const std::size_t n)
-        {
-                if (size_ < n)
-                {
-                        allocate(n);
-                }
-        }
-
         void upload(const std::vector<X>& v)
         {
                 allocate(v.size());
@@ -2828,7 +2819,6 @@ public:
                 {
                         state_.allocate(pixels_);
                 }
-                groups_.allocate(group_bytes(pixels_, spp_, double_sums_));
                 stats_.allocate(1);
                 NBPT_CUDA(cudaMemsetAsync(stats_.get(), 0, sizeof(PathStats), stream_));
                 cancel_.allocate(1);
@@ -2844,6 +2834,7 @@ public:
                 chunk_pixels_ = chunk_pixels(sources_, spp_, max_depth_, integrator_, chunk_budget_);
                 if (integrator_ == Integrator::PT)
                 {
+                        groups_.allocate(group_bytes(pixels_, spp_, double_sums_));
                         next_path_.allocate(1);
                         // as many blocks as the device holds at once
                         const std::size_t shared = wide_stack_bytes<T>(scene_->device().wide_stack, PT_THREADS);
@@ -3006,7 +2997,8 @@ public:
                 }
         }
 
-        // the per-chunk buffers of the BPT path kernels
+        // the per-chunk buffers of the BPT path kernels and the accumulation's
+        // groups: what release_scratch() gives back
         void allocate_scratch()
         {
                 const long long paths = chunk_pixels_ * spp_;
@@ -3015,6 +3007,7 @@ public:
                 rng_.allocate(paths);
                 queues_.allocate(queue_bytes(paths, max_depth_));
                 arrivals_.allocate(paths * max_depth_);
+                groups_.allocate(group_bytes(pixels_, spp_, double_sums_));
                 scratch_ready_ = true;
         }
 
@@ -3300,8 +3293,6 @@ public:
                         return;
                 }
                 const long long range = group_pixels<S>(pixels_);
-                // release_scratch() gives it back (of a render that a job server made)
-                groups_.allocate_if_smaller(group_bytes(pixels_, spp_, double_sums_));
                 auto* const groups = reinterpret_cast<PixelState<3, S>*>(groups_.get());
                 long long reach = 0;
                 long long row = 1;
