@@ -212,14 +212,19 @@ def cpu_baseline(small: bool, name: str = "cornell4d", precision: str = "float",
                        f"({paths} paths, {seconds:.2f} s)")}
 
 
-# DRAM bytes (read + write) per path of the path kernels (walk, connect,
-# light, replay) on this workload in float, from the ncu capture summarised
+# DRAM bytes (read + write) per path of the path kernels (walk, light, connect,
+# sight, replay) on this workload in float, from the ncu capture summarised
 # in profiles/path_kernels_cornell4d_32.md (a 32^3 screen of the same scene;
 # traffic scales with the number of paths)
-TRAFFIC_PER_PATH = {"float": 20636.0}
+TRAFFIC_PER_PATH = {"float": 5290.0}
 
 
 def record_bytes(n: int, precision: str) -> dict:
+    """Bytes of a tested BVH box with its two words (a child of an eight-child
+    node; its alignment not counted), of a facet's planes and of a shape.  The
+    statistics' `nodes` counts boxes: the children of every node visited, where
+    a binary walk counts one box per node (46.3 and 40.0 per path of the mixed
+    batch), so bytes of earlier lines, from binary nodes, are some 4 % lower."""
     t = 8 if precision == "double" else 4
     return {"node": 2 * n * t + 8, "facet": n * (n + 1) * t + 4, "shape": n * (n + 1) * t}
 
@@ -409,7 +414,7 @@ def run_nbpt(args, rank: int, world: int, local: int):
                             if args.precision in TRAFFIC_PER_PATH and args.workload == "cornell4d"
                             and args.integrator == "bpt" and not args.small and args.screen is None else None),
                 "traffic_source": "profiles/path_kernels_cornell4d_32.md (per path, scaled to one pass)",
-                "kernel": ("path kernels (walk, connect, light, replay)" if args.integrator == "bpt"
+                "kernel": ("path kernels (walk, light, connect, sight, replay)" if args.integrator == "bpt"
                            else "pt_paths_kernel"),
                 "peak_source": "measured" if "hbm_gbs" in peaks else "fallback",
                 "algorithmic_bytes_per_path": algorithmic / (paths_per_step * args.steps),
