@@ -23,9 +23,8 @@ struct FloatPathKernels final
         decltype(&connect_sight_kernel<N, float>) sight;
         decltype(&paths_replay_kernel<N, float, 3, 1>) replay_rgb;
         decltype(&paths_replay_kernel<N, float, 64, 32>) replay_spectrum;
-        // [many_shapes()]
-        decltype(&pt_paths_kernel<N, float, 3, false>) pt_rgb[2];
-        decltype(&pt_paths_kernel<N, float, 64, false>) pt_spectrum[2];
+        PtKernels<N, float, 3> pt_rgb;
+        PtKernels<N, float, 64> pt_spectrum;
 };
 
 template <int N>

@@ -2838,9 +2838,10 @@ public:
                         next_path_.allocate(1);
                         // as many blocks as the device holds at once
                         const std::size_t shared = wide_stack_bytes<T>(scene_->device().wide_stack, PT_THREADS);
-                        allow_shared(pt_kernel(), shared);
+                        const auto kernel = pt_kernel(chunk_pixels_ * spp_);
+                        allow_shared(kernel, shared);
                         int resident = 0;
-                        NBPT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, pt_kernel(), PT_THREADS, shared));
+                        NBPT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, kernel, PT_THREADS, shared));
                         connect_blocks_ = sms * std::max(1, resident);
                         // direct-lighting records: 2 per light per thread
                         pt_estimates_.allocate(std::max(1LL, static_cast<long long>(connect_blocks_) * PT_THREADS * 2 *
@@ -2976,24 +2977,25 @@ public:
                         return &paths_replay_kernel<N, T, C, LANES>;
                 }
         }
-        auto pt_kernel() const
+        // the PT kernel of a chunk of this many paths
+        auto pt_kernel(const long long paths) const
         {
-                const bool many = many_shapes(scene_->device());
+                const DeviceScene<N, T, 1>& scene = scene_->device_channel_0();
                 if constexpr (std::is_same_v<T, float>)
                 {
                         static_assert(C == 3 || C == 64);
                         if constexpr (C == 3)
                         {
-                                return float_path_kernels<N>().pt_rgb[many];
+                                return float_path_kernels<N>().pt_rgb.of(scene, paths);
                         }
                         else
                         {
-                                return float_path_kernels<N>().pt_spectrum[many];
+                                return float_path_kernels<N>().pt_spectrum.of(scene, paths);
                         }
                 }
                 else
                 {
-                        return many ? &pt_paths_kernel<N, T, C, true> : &pt_paths_kernel<N, T, C, false>;
+                        return PT_KERNELS<N, T, C>.of(scene, paths);
                 }
         }
 
@@ -3085,7 +3087,7 @@ public:
                                         const long long o = b - source_first_; // the chunk in the sample arrays
                                         const long long n = (e - b) * spp_;
                                         NBPT_CUDA(cudaMemsetAsync(next_path_.get(), 0, sizeof(unsigned), stream_));
-                                        pt_kernel()
+                                        pt_kernel(chunk_pixels_ * spp_)
                                                 <<<std::min<long long>(connect_blocks_, blocks_for(n, PT_THREADS)), PT_THREADS,
                                                    wide_stack_bytes<T>(scene_1.wide_stack, PT_THREADS), stream_>>>(
                                                         scene_1, scene_->device_materials(),

@@ -14,8 +14,7 @@ const FloatPathKernels<N>& float_path_kernels()
                 &paths_connect_kernel<N, float>,       &connect_sight_kernel<N, float>,
                 &paths_replay_kernel<N, float, 3, 1>,
                 &paths_replay_kernel<N, float, 64, 32>,
-                {&pt_paths_kernel<N, float, 3, false>, &pt_paths_kernel<N, float, 3, true>},
-                {&pt_paths_kernel<N, float, 64, false>, &pt_paths_kernel<N, float, 64, true>}};
+                PT_KERNELS<N, float, 3>,               PT_KERNELS<N, float, 64>};
         return kernels;
 }
 
