@@ -251,30 +251,25 @@ __device__ float pt_brdf_channel(const BrdfTerms& t, const int zero, const Mater
 // the output row.  `estimates` holds 2 * light_count records per thread of
 // the grid.
 //
-// Paths whose primary ray meets nothing are over at once: a warp goes on
-// starting paths until fewer than PT_REFILL of its lanes are without one, so
-// that the rest of the bounce has lanes to work on (3-space, 5 % of the primary
-// rays hit: 0.48 -> 0.39 ms per 1.0 M paths; where most hit, no difference; 4
-// instead of 8 is 1 to 2 % slower).
-//
-// BLOCKS per SM cap the registers (65536 / (256 * BLOCKS)), IN_STEP is whether
-// a block's warps meet at the barriers.  A scene of nothing but a mesh, whose
-// primary rays all look for a facet and whose paths mostly end there, spends its
-// time in queries that wait for memory and at barriers after the longest of
-// them: more blocks, and in single precision none in step (4-space mesh of 20,000
-// points, 3.4 M paths, 30 % hit, single precision: 2 blocks in step 14.3 ms, 4
-// 10.6, 5 10.0, 4 not in step 8.7; double 18.9, with 3 blocks 17.0, not in step
-// 20.3), from as many paths on as fill them (0.37 M paths 2.2 -> 1.5 and 2.8 ->
-// 2.7 ms; 0.22 M 1.33 and 1.37).  Not in 5-space, where hardly a primary ray
-// hits (1.7 M paths 2.3 and 2.5 ms).
+// A scene of nothing but a mesh, whose primary rays all look for a facet and
+// whose paths mostly end there, spends its time in queries that wait for memory
+// and at barriers after the longest of them.  From as many paths on as fill them
+// it takes kernels of more blocks per SM (with fewer registers for it), in single
+// precision not in step either (IN_STEP), whose warps go on starting paths until
+// fewer than PT_REFILL of their lanes are without one that hit something (REFILL).
+// 4-space mesh of 20,000 points, 3.4 M paths, 30 % hit, single precision: 2 blocks
+// in step 14.3 ms, 4 10.6, 5 10.0, 4 not in step 8.7; double 18.9, with 3 blocks
+// 17.0, not in step 20.3; 0.37 M paths 2.2 -> 1.5 and 2.8 -> 2.7; 0.22 M the same.
+// Not in 5-space, where hardly a primary ray hits (1.7 M paths 2.3 and 2.5 ms);
+// and with walls, which most rays hit, starting anew gains nothing and costs the
+// small renders registers (5-space, single precision, 20,000 paths 1.1 -> 1.3).
 inline constexpr int PT_THREADS = 256;
-inline constexpr int PT_REFILL = 8;
-inline constexpr int PT_BLOCKS = 2;
+inline constexpr int PT_REFILL = 16;
 inline constexpr long long PT_MESH_PATHS = 300'000;
 
-template <int N, typename T, int C, bool MANY, int BLOCKS, bool IN_STEP>
-__global__ void __launch_bounds__(PT_THREADS, BLOCKS) pt_paths_kernel(
-        const DeviceScene<N, T, 1> scene,
+template <int N, typename T, int C, bool MANY, bool REFILL, bool IN_STEP>
+__device__ __forceinline__ void pt_paths(
+        const DeviceScene<N, T, 1>& scene,
         const Material<T, C>* __restrict__ materials,
         const Light<N, T, C>* __restrict__ lights,
         const long long begin,
@@ -312,6 +307,50 @@ __global__ void __launch_bounds__(PT_THREADS, BLOCKS) pt_paths_kernel(
         int depth = STARTS; // the bounce whose hit is traced next; -1: the primary ray, STARTS: a path to be started
         long long i = -1; // the lane's path; -1 when it takes the next one
         bool done = false;
+        const auto take_path = [&]
+        {
+                i = cancelled(cancel) ? paths : reserve_together(next_path, 1);
+                done = i >= paths;
+                i = done ? -1 : i;
+        };
+        const auto start_path = [&]
+        {
+                // 32-bit index arithmetic: a chunk's path index and a
+                // screen's pixel index fit in 31 bits (the painter's chunk
+                // limits and its screen check), and a 64-bit division costs
+                // several times a 32-bit one
+                const unsigned local_pixel = static_cast<unsigned>(i) / static_cast<unsigned>(spp);
+                const int sample = static_cast<int>(static_cast<unsigned>(i) - local_pixel * spp);
+                const unsigned p = static_cast<unsigned>(begin) + local_pixel;
+                Vec<N - 1, T> point;
+                {
+                        unsigned rest = p;
+#pragma unroll
+                        for (int d = 0; d < N - 1; ++d)
+                        {
+                                const unsigned size = static_cast<unsigned>(scene.projector.size[d]);
+                                const unsigned r = rest / size;
+                                point[d] = static_cast<T>(static_cast<int>(rest - r * size)) +
+                                           points[i * (N - 1) + d];
+                                rest = r;
+                        }
+                }
+                ray = scene.projector.ray(point);
+                const std::uint32_t words[4] = {seed, pass, static_cast<std::uint32_t>(p),
+                                                static_cast<std::uint32_t>(sample + 1)};
+                g = seed_seq_pcg(words, 4);
+                depth = -1;
+        };
+        const auto write_background = [&]
+        {
+#pragma unroll 8
+                for (int c = 0; c < C; ++c)
+                {
+                        colors[i * C + c] = 0.0f;
+                }
+                lum[i] = 0.0f;
+                valid[i] = 0;
+        };
         const auto in_step = []
         {
                 if constexpr (IN_STEP)
@@ -322,80 +361,75 @@ __global__ void __launch_bounds__(PT_THREADS, BLOCKS) pt_paths_kernel(
         while (true)
         {
                 Hit<N, T> surface;
-                surface.kind = static_cast<int>(HitKind::NONE);
                 Normals<N, T> normals;
-                bool traced = false;
-                in_step();
-                while (true)
+                bool background = false; // written already
+                if constexpr (!REFILL)
                 {
                         if (i < 0 && !done)
                         {
-                                i = cancelled(cancel) ? paths : reserve_together(next_path, 1);
-                                done = i >= paths;
-                                i = done ? -1 : i;
+                                take_path();
                         }
-                        const bool fresh = i >= 0 && !traced;
-                        if (fresh && depth == STARTS)
+                        if (__syncthreads_and(done ? 1 : 0) != 0)
                         {
-                                // 32-bit index arithmetic: a chunk's path index and a
-                                // screen's pixel index fit in 31 bits (the painter's chunk
-                                // limits and its screen check), and a 64-bit division costs
-                                // several times a 32-bit one
-                                const unsigned local_pixel = static_cast<unsigned>(i) / static_cast<unsigned>(spp);
-                                const int sample = static_cast<int>(static_cast<unsigned>(i) - local_pixel * spp);
-                                const unsigned p = static_cast<unsigned>(begin) + local_pixel;
-                                Vec<N - 1, T> point;
+                                break;
+                        }
+                        if (i >= 0 && depth == STARTS)
+                        {
+                                start_path();
+                        }
+                        surface = warp.scene_intersect(i >= 0, depth >= 0, gn, ray, normals);
+                        __syncthreads();
+                        background = i >= 0 && depth < 0 && !surface;
+                        if (background)
+                        {
+                                write_background();
+                        }
+                }
+                else
+                {
+                        surface.kind = static_cast<int>(HitKind::NONE);
+                        bool traced = false;
+                        in_step();
+                        while (true)
+                        {
+                                if (i < 0 && !done)
                                 {
-                                        unsigned rest = p;
-#pragma unroll
-                                        for (int d = 0; d < N - 1; ++d)
+                                        take_path();
+                                }
+                                const bool fresh = i >= 0 && !traced;
+                                if (fresh && depth == STARTS)
+                                {
+                                        start_path();
+                                }
+                                Normals<N, T> found;
+                                const Hit<N, T> hit = warp.scene_intersect(fresh, depth >= 0, gn, ray, found);
+                                if (fresh)
+                                {
+                                        surface = hit;
+                                        normals = found;
+                                        traced = true;
+                                        if (depth < 0 && !hit)
                                         {
-                                                const unsigned size = static_cast<unsigned>(scene.projector.size[d]);
-                                                const unsigned r = rest / size;
-                                                point[d] = static_cast<T>(static_cast<int>(rest - r * size)) +
-                                                           points[i * (N - 1) + d];
-                                                rest = r;
+                                                write_background();
+                                                i = -1;
+                                                depth = STARTS;
+                                                traced = false;
                                         }
                                 }
-                                ray = scene.projector.ray(point);
-                                const std::uint32_t words[4] = {seed, pass, static_cast<std::uint32_t>(p),
-                                                                static_cast<std::uint32_t>(sample + 1)};
-                                g = seed_seq_pcg(words, 4);
-                                depth = -1;
-                        }
-                        Normals<N, T> found;
-                        const Hit<N, T> hit = warp.scene_intersect(fresh, depth >= 0, gn, ray, found);
-                        if (fresh)
-                        {
-                                surface = hit;
-                                normals = found;
-                                traced = true;
-                                if (depth < 0 && !hit)
+                                if (__popc(__ballot_sync(W::FULL, i < 0 && !done)) < PT_REFILL)
                                 {
-#pragma unroll 8
-                                        for (int c = 0; c < C; ++c)
-                                        {
-                                                colors[i * C + c] = 0.0f;
-                                        }
-                                        lum[i] = 0.0f;
-                                        valid[i] = 0;
-                                        i = -1;
-                                        depth = STARTS;
-                                        traced = false;
+                                        break;
                                 }
                         }
-                        if (__popc(__ballot_sync(W::FULL, i < 0 && !done)) < PT_REFILL)
+                        if (IN_STEP ? __syncthreads_and(i < 0 && done ? 1 : 0) != 0
+                                    : __all_sync(W::FULL, i < 0 && done) != 0)
                         {
                                 break;
                         }
                 }
-                if (IN_STEP ? __syncthreads_and(i < 0 && done ? 1 : 0) != 0 : __all_sync(W::FULL, i < 0 && done) != 0)
-                {
-                        break;
-                }
                 const bool live = i >= 0;
                 float* const out = colors + i * C;
-                if (live && depth < 0)
+                if (live && !background && depth < 0)
                 {
                         // the emitted radiance seen by the primary ray
                         // (LightSource::leave_radiance(-dir))
@@ -420,7 +454,7 @@ __global__ void __launch_bounds__(PT_THREADS, BLOCKS) pt_paths_kernel(
 
                 // one bounce (pt.cpp:68-111); the path ends where the
                 // reference's loop breaks
-                bool go_on = live && static_cast<bool>(surface);
+                bool go_on = live && !background && static_cast<bool>(surface);
                 const Vec<N, T> v = -ray.dir;
                 if (go_on)
                 {
@@ -538,6 +572,10 @@ __global__ void __launch_bounds__(PT_THREADS, BLOCKS) pt_paths_kernel(
                 const long long path = i;
                 i = -1;
                 depth = STARTS;
+                if (background)
+                {
+                        continue;
+                }
 
                 // the path is done
                 if constexpr (IN_REGISTERS)
@@ -572,12 +610,61 @@ __global__ void __launch_bounds__(PT_THREADS, BLOCKS) pt_paths_kernel(
         add_counters(counters, stats);
 }
 
+template <int N, typename T, int C, bool MANY>
+__global__ void __launch_bounds__(PT_THREADS) pt_paths_kernel(
+        const DeviceScene<N, T, 1> scene,
+        const Material<T, C>* __restrict__ materials,
+        const Light<N, T, C>* __restrict__ lights,
+        const long long begin,
+        const long long end,
+        const int spp,
+        const std::uint32_t seed,
+        const std::uint32_t pass,
+        const T* __restrict__ points,
+        float* __restrict__ colors,
+        float* __restrict__ lum,
+        unsigned char* __restrict__ valid,
+        PtEstimate* __restrict__ estimates,
+        unsigned* __restrict__ next_path,
+        PathStats* __restrict__ stats,
+        const float* __restrict__ cie_y,
+        const unsigned* __restrict__ cancel)
+{
+        pt_paths<N, T, C, MANY, false, true>(scene, materials, lights, begin, end, spp, seed, pass, points, colors, lum,
+                                             valid, estimates, next_path, stats, cie_y, cancel);
+}
+
+// Scenes of one mesh and nothing else (see above).
+template <int N, typename T, int C>
+__global__ void __launch_bounds__(PT_THREADS, (sizeof(T) == 4 ? 4 : 3)) pt_mesh_paths_kernel(
+        const DeviceScene<N, T, 1> scene,
+        const Material<T, C>* __restrict__ materials,
+        const Light<N, T, C>* __restrict__ lights,
+        const long long begin,
+        const long long end,
+        const int spp,
+        const std::uint32_t seed,
+        const std::uint32_t pass,
+        const T* __restrict__ points,
+        float* __restrict__ colors,
+        float* __restrict__ lum,
+        unsigned char* __restrict__ valid,
+        PtEstimate* __restrict__ estimates,
+        unsigned* __restrict__ next_path,
+        PathStats* __restrict__ stats,
+        const float* __restrict__ cie_y,
+        const unsigned* __restrict__ cancel)
+{
+        pt_paths<N, T, C, false, true, sizeof(T) == 8>(scene, materials, lights, begin, end, spp, seed, pass, points,
+                                                       colors, lum, valid, estimates, next_path, stats, cie_y, cancel);
+}
+
 // The kernels of a dimension, precision and colour, by scene and paths of a
 // chunk.
 template <int N, typename T, int C>
 struct PtKernels final
 {
-        using Kernel = decltype(&pt_paths_kernel<N, T, C, false, PT_BLOCKS, true>);
+        using Kernel = decltype(&pt_paths_kernel<N, T, C, false>);
         Kernel ordinary;
         Kernel meshes;
         Kernel many;
@@ -596,19 +683,15 @@ template <int N, typename T, int C>
 constexpr PtKernels<N, T, C> pt_kernels()
 {
         PtKernels<N, T, C> k{};
-        k.ordinary = &pt_paths_kernel<N, T, C, false, PT_BLOCKS, true>;
-        k.many = &pt_paths_kernel<N, T, C, true, PT_BLOCKS, true>;
+        k.ordinary = &pt_paths_kernel<N, T, C, false>;
+        k.many = &pt_paths_kernel<N, T, C, true>;
         if constexpr (N == 5)
         {
                 k.meshes = k.ordinary;
         }
-        else if constexpr (sizeof(T) == 4)
-        {
-                k.meshes = &pt_paths_kernel<N, T, C, false, 4, false>;
-        }
         else
         {
-                k.meshes = &pt_paths_kernel<N, T, C, false, 3, true>;
+                k.meshes = &pt_mesh_paths_kernel<N, T, C>;
         }
         return k;
 }
